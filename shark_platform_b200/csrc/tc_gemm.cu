@@ -29,13 +29,17 @@
 //               tensor-memory store latency hides behind the other's arithmetic
 //   warp  16    TMA producer for weights and scales
 //   warp  17    TMA producer for token tiles
-//   warp  18    TMEM allocation; one lane issues the MMAs of row set 0 and commits
-//   warp  19    one lane issues the MMAs of row set 1
-// Two issuers because issuing is what the loop is short of: an MMA costs its
-// issuing thread ~70 clocks, eight per 64-k stage plus the barrier waits exceed
-// the 768 clocks the tensor pipe needs for them, so with one issuer the pipe runs
-// dry every stage.  Each row set has its own A-slot barriers, so the two sets
-// are independent pipelines that share only the token tiles.
+//   warp  18    TMEM allocation; issues the MMAs of row set 0 and commits
+//   warp  19    issues the MMAs of row set 1
+// The MMAs are issued by an elected lane (elect.sync) of a converged warp.  Issued
+// under `if (lane == 0)` instead, an MMA costs its thread ~70 clocks and the loop
+// took 1055 clocks per 64-k stage where the tensor pipe needs 704: the compiler
+// cannot know that one lane is active and guards the instruction's uniform
+// operands.  Measured, one B200, us per launch, gate/up + down: 4096 tokens Q8_0
+// 1618 + 873 -> 1500 + 804, 2048 tokens Q4_K 942 + 482 -> 840 + 428, 128 tokens Q8_0
+// 250 + 129 -> 209 + 110.
+// Each row set has its own A-slot barriers, so the two sets are independent
+// pipelines that share only the token tiles.
 //
 // Tensor-memory columns (512 allocated): accumulators at 0 and 192 (192 fp32
 // columns each), two A staging slots of 2 x 32 columns at 384..511.
@@ -252,7 +256,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const uint32_t a_ready = take(2 * TC_ASLOTS), a_free = take(2 * TC_ASLOTS);  // [slot][row set]
   const uint32_t acc_full_bar = take(1), acc_empty_bar = take(1);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // the shuffle tells the compiler that the warp index is warp-uniform
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (tid == 0) {
     s_abort = 0;
     for (int s = 0; s < TC_WSLOTS; ++s) {
@@ -398,44 +403,43 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     }
   } else if (warp == TC_WARP_MMA || warp == TC_WARP_MMA1) {
     // ------------------------------------------ MMA issuers, one per row set
-    if (lane == 0) {
-      const int mset = warp - TC_WARP_MMA;
-      const uint32_t acc = tmem + (mset == 0 ? TC_COL_ACC0 : TC_COL_ACC1);
-      uint32_t ti = 0;
-      bool ok = true;
-      // slot indices and phase parities advance by counters: this lane's
-      // instruction stream is the kernel's critical path (every instruction of
-      // it was measured at 15-20 clocks beside the sixteen dequantising warps)
-      uint32_t xs = 0, xph = 0, as = 0, aph = 0;
-      static_assert(TC_KT == 64, "tc_mma_ts_x4 issues the four K steps of a 64-k stage");
-      const uint32_t desc_hi = static_cast<uint32_t>(smem_desc_sw128(0) >> 32);
-      const uint32_t a_set = tmem + TC_COL_A + mset * 32;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++ti) {
-        int e, nt, row0, rows, ncols;
-        decode(tile, e, nt, row0, rows, ncols);
-        const uint32_t idesc = make_idesc(128, ncols);
-        if (!mbar_wait(acc_empty_bar, (ti & 1u) ^ 1u, abort_flag, args.status)) break;
+    const int mset = warp - TC_WARP_MMA;
+    const uint32_t acc = tmem + (mset == 0 ? TC_COL_ACC0 : TC_COL_ACC1);
+    uint32_t ti = 0;
+    bool ok = true;
+    uint32_t xs = 0, xph = 0, as = 0, aph = 0;
+    static_assert(TC_KT == 64, "tc_mma_ts_x4 issues the four K steps of a 64-k stage");
+    const uint32_t desc_hi = static_cast<uint32_t>(smem_desc_sw128(0) >> 32);
+    const uint32_t a_set = tmem + TC_COL_A + mset * 32;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++ti) {
+      int e, nt, row0, rows, ncols;
+      decode(tile, e, nt, row0, rows, ncols);
+      const uint32_t idesc = make_idesc(128, ncols);
+      if (!mbar_wait_warp(acc_empty_bar, (ti & 1u) ^ 1u, abort_flag, args.status)) break;
+      tc_fence_after();
+      for (int st = 0; st < stages_per_tile; ++st) {
+        const uint32_t ab = 8u * (2 * as + mset);
+        const uint32_t sub = static_cast<uint32_t>(st) & 1u;  // half of the token slot (tiles hold an even number of stages)
+        if ((sub == 0 && !mbar_wait_warp(xfull + 8u * xs, xph, abort_flag, args.status)) ||
+            !mbar_wait_warp(a_ready + ab, aph, abort_flag, args.status)) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        for (int st = 0; st < stages_per_tile; ++st) {
-          const uint32_t ab = 8u * (2 * as + mset);
-          const uint32_t sub = static_cast<uint32_t>(st) & 1u;  // half of the token slot (tiles hold an even number of stages)
-          if ((sub == 0 && !mbar_wait(xfull + 8u * xs, xph, abort_flag, args.status)) ||
-              !mbar_wait(a_ready + ab, aph, abort_flag, args.status)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t b_lo = ((x_base + xs * TC_XSLOT + sub * TC_XSUB) & 0x3FFFFu) >> 4;
+        const uint32_t b_lo = ((x_base + xs * TC_XSLOT + sub * TC_XSUB) & 0x3FFFFu) >> 4;
+        if (elect_one()) {
           tc_mma_ts_x4(acc, a_set + as * 64, b_lo, desc_hi, idesc, st > 0 ? 1u : 0u);
           tc_commit(a_free + ab);
-          if (sub) {
-            tc_commit(xempty + 8u * xs);
-            if (++xs == TC_XSLOTS) { xs = 0; xph ^= 1u; }
-          }
-          if (++as == TC_ASLOTS) { as = 0; aph ^= 1u; }
+          if (sub) tc_commit(xempty + 8u * xs);
         }
-        if (ok) tc_commit(acc_full_bar);
+        __syncwarp();
+        if (sub) {
+          if (++xs == TC_XSLOTS) { xs = 0; xph ^= 1u; }
+        }
+        if (++as == TC_ASLOTS) { as = 0; aph ^= 1u; }
       }
+      if (ok && elect_one()) tc_commit(acc_full_bar);
+      __syncwarp();
     }
   } else {
     // ------------------------------------- dequantise (both sets) + epilogue
