@@ -110,14 +110,17 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // DEV_ERR_WAIT_TIMEOUT in the status word and raises the CTA-wide abort flag so
 // that every later wait in this CTA returns at once.  Returns false on abort.
 // The barrier is tried first: a phase that has already completed costs one
-// try_wait and no shared-memory load of the abort flag.
+// try_wait and no shared-memory load of the abort flag.  A waiting warp polls the
+// barrier alone and looks at the flag and the clock on every 32nd poll only: the
+// GEMM kernels are short of issue slots, and polls take them from working warps.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int32_t* status) {
   if (mbar_try_wait(bar, parity)) return true;
-  if (*abort_flag) return false;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i)
+      if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     if (clock64() - t0 > (1ll << 31)) {
       *abort_flag = 1;
@@ -205,23 +208,26 @@ __device__ __forceinline__ void dequant_q8x4(uint32_t w, __half2 scale, uint32_t
 // Eight 4-bit quants of one 32-bit word (k order: nibble i of byte b is
 // element 2b+i) -> fp16(fp16(ds*q) - dm) as four half2 whose element pairs are
 // (q0,q4) (q1,q5) (q2,q6) (q3,q7): the pair order the activation rows are
-// pre-permuted to.  0x6400|q is the fp16 number 1024+q, and -1024*ds is exact in
-// fp16 (a power-of-two multiple; ds < 64), so one fused multiply-add
-// (1024+q)*ds - 1024*ds is the exact product ds*q rounded once — the value of the
-// reference's fp16 multiply — without first subtracting the 1024.  The offset is
-// then subtracted with its own rounding (_rn: never contracted into the fma).
+// pre-permuted to.  A nibble in bits 0-3 under 0x6400 is the fp16 number 1024+q;
+// one in bits 4-7 under 0x5400 is 64+q, so the odd nibbles need no shift.  -1024*ds
+// and -64*ds are exact in fp16 (power-of-two multiples; ds < 64), so one fused
+// multiply-add (1024+q)*ds - 1024*ds (or with 64) is the exact product ds*q rounded
+// once — the value of the reference's fp16 multiply — without first subtracting the
+// offset.  dm is then subtracted with its own rounding (_rn: never contracted into
+// the fma).  13 instructions per eight weights; shifting all odd nibbles down took 15.
 __device__ __forceinline__ void dequant_q4x8(uint32_t w, __half2 ds, __half2 dm,
                                              uint32_t (&out)[4]) {
   const __half2 nds1024 = __hmul2(ds, u32_as_h2(0xE400E400u));  // -1024 * ds, exact
+  const __half2 nds64 = __hmul2(ds, u32_as_h2(0xD400D400u));    // -64 * ds, exact
   const uint32_t w1 = w >> 8;
   uint32_t e[4];
-  e[0] = (w & 0x000f000fu) | 0x64006400u;          // (q0, q4)
-  e[1] = ((w >> 4) & 0x000f000fu) | 0x64006400u;   // (q1, q5)
-  e[2] = (w1 & 0x000f000fu) | 0x64006400u;         // (q2, q6)
-  e[3] = ((w1 >> 4) & 0x000f000fu) | 0x64006400u;  // (q3, q7)
+  e[0] = (w & 0x000f000fu) | 0x64006400u;   // (q0, q4) + 1024
+  e[1] = (w & 0x00f000f0u) | 0x54005400u;   // (q1, q5) + 64
+  e[2] = (w1 & 0x000f000fu) | 0x64006400u;  // (q2, q6) + 1024
+  e[3] = (w1 & 0x00f000f0u) | 0x54005400u;  // (q3, q7) + 64
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const __half2 t = __hfma2(u32_as_h2(e[i]), ds, nds1024);
+    const __half2 t = __hfma2(u32_as_h2(e[i]), ds, (i & 1) ? nds64 : nds1024);
     out[i] = h2_as_u32(__hsub2_rn(t, dm));
   }
 }

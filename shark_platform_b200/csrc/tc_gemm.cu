@@ -46,6 +46,8 @@
 //
 // All mbarrier waits are bounded; on expiry the CTA raises its abort flag, every
 // role falls out of its loops, the CTA frees its tensor memory and returns.
+#include <math.h>
+
 #include "common.cuh"
 
 namespace b200moe {
@@ -77,7 +79,12 @@ constexpr int TC_SSLOT = 2 * TC_SSET;
 template <int NMAX>
 struct TcCfg {
   static_assert(NMAX == 64 || NMAX == 128 || NMAX == 192, "token tile widths: 64, 128, 192");
-  static constexpr int ASLOTS = (512 - 2 * NMAX) / 64;  // 6, 4, 2 (even: a slot belongs to one dequant group)
+  static constexpr int ASLOTS = (512 - 2 * NMAX) / 64;  // 6, 4, 2 stages of 64 k
+  // stages per hand-over from the dequant warps to the issuers: two where the ring
+  // holds more than two, which halves the waits, votes, fences and arrivals per
+  // weight on both sides
+  static constexpr int HK = NMAX <= 128 ? 2 : 1;
+  static constexpr int HSLOTS = ASLOTS / HK;            // 3, 2, 2
   static constexpr int WSLOTS = NMAX == 192 ? 2 : NMAX == 128 ? 3 : 5;
   // a token slot holds two 64-k stages (two swizzled sub-tiles of NMAX rows x 128 B):
   // one wait and one release per 128 k on the issuing lanes, whose instruction
@@ -92,13 +99,14 @@ struct TcCfg {
   static constexpr uint32_t COL_ACC0 = 0, COL_ACC1 = NMAX, COL_A = 2 * NMAX;
   static_assert(XSLOT % 1024 == 0 && TC_WSLOT % 1024 == 0, "slot alignment for the swizzle");
   static_assert(SMEM <= 232448, "shared memory budget");
-  static_assert(2 * (WSLOTS + XSLOTS + TC_SSLOTS + 2 * ASLOTS) + 2 <= 64, "barrier area");
+  static_assert(2 * (WSLOTS + XSLOTS + TC_SSLOTS + 2 * HSLOTS) + 2 <= 64, "barrier area");
 };
 
 struct TcArgs {
   const int32_t* seg;
   int E, N, K;
-  int ntiles;      // row tiles per expert (N / 128 for gate+up, N / 256 for down)
+  int row_tile;    // weight rows per set (<= 128, a multiple of 16): tc_row_tile
+  int ntiles;      // row tiles per expert (N / row_tile for gate+up, N / 256 for down)
   int tok_tile;    // upper bound on tokens per tile (multiple of 16, <= 192)
   int ksplit;      // k partitions per tile (down only); partial kc goes to out + kc*P*N
   int P;
@@ -242,7 +250,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   __shared__ uint32_t s_tmem;
 
   using G = TcCfg<NMAX>;
-  constexpr int TC_WSLOTS = G::WSLOTS, TC_XSLOTS = G::XSLOTS, TC_XSLOT = G::XSLOT, TC_XSUB = G::XSUB, TC_ASLOTS = G::ASLOTS;
+  constexpr int TC_WSLOTS = G::WSLOTS, TC_XSLOTS = G::XSLOTS, TC_XSLOT = G::XSLOT, TC_XSUB = G::XSUB, HK = G::HK, HSLOTS = G::HSLOTS;
   constexpr uint32_t TC_COL_ACC0 = G::COL_ACC0, TC_COL_ACC1 = G::COL_ACC1, TC_COL_A = G::COL_A;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t x_base = smem_base + G::OFF_X;
@@ -253,7 +261,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const uint32_t wfull = take(TC_WSLOTS), wempty = take(TC_WSLOTS);
   const uint32_t xfull = take(TC_XSLOTS), xempty = take(TC_XSLOTS);
   const uint32_t sfull = take(TC_SSLOTS), sempty = take(TC_SSLOTS);
-  const uint32_t a_ready = take(2 * TC_ASLOTS), a_free = take(2 * TC_ASLOTS);  // [slot][row set]
+  const uint32_t a_ready = take(2 * HSLOTS), a_free = take(2 * HSLOTS);  // [slot][row set]
   const uint32_t acc_full_bar = take(1), acc_empty_bar = take(1);
 
   // the shuffle tells the compiler that the warp index is warp-uniform
@@ -262,7 +270,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     s_abort = 0;
     for (int s = 0; s < TC_WSLOTS; ++s) {
       mbar_init(wfull + 8u * s, 1);
-      mbar_init(wempty + 8u * s, TC_DQ_WARPS);
+      mbar_init(wempty + 8u * s, HK == 2 ? TC_DQ_WARPS / 2 : TC_DQ_WARPS);  // the warps that read the slot
     }
     for (int s = 0; s < TC_XSLOTS; ++s) {
       mbar_init(xfull + 8u * s, 1);
@@ -272,7 +280,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       mbar_init(sfull + 8u * s, 1);
       mbar_init(sempty + 8u * s, TC_DQ_WARPS);
     }
-    for (int s = 0; s < 2 * TC_ASLOTS; ++s) {
+    for (int s = 0; s < 2 * HSLOTS; ++s) {
       mbar_init(a_ready + 8u * s, TC_DQ_WARPS / 4);  // one arrival per warp of the group and row set that fills it
       mbar_init(a_free + 8u * s, 1);
     }
@@ -301,8 +309,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   volatile int* abort_flag = &s_abort;
   const int stages_per_tile = args.K / TC_KT / args.ksplit;  // a multiple of 4
   constexpr bool Q4 = LAYOUT == B200MOE_LAYOUT_Q4_K;
-  constexpr uint32_t WSET_BYTES = Q4 ? TC_ROWS * 64 : TC_ROWS * 128;  // one set, 128 k
-  constexpr uint32_t SSET_BYTES = Q4 ? TC_ROWS * 32 : TC_ROWS * 16;   // one set, 256 k
+  const uint32_t set_rows = static_cast<uint32_t>(args.row_tile);
+  const uint32_t WSET_BYTES = set_rows * (Q4 ? 64 : 128);  // one set, 128 k
+  const uint32_t SSET_BYTES = set_rows * (Q4 ? 32 : 16);   // one set, 256 k
 
   // tile -> (expert, row tile | k partition << 16, first token row, token rows, MMA N)
   auto decode = [&](int tile, int& e, int& nt, int& row0, int& rows, int& ncols) {
@@ -331,7 +340,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         decode(tile, e, nt, row0, rows, ncols);
         const int kbase = (nt >> 16) * stages_per_tile * TC_KT;
         nt &= 0xffff;
-        const int grow0 = e * args.N + nt * (NMAT == 2 ? TC_ROWS : 2 * TC_ROWS);
+        const int grow0 = e * args.N + nt * (NMAT == 2 ? args.row_tile : 2 * TC_ROWS);
         const int grow1 = NMAT == 2 ? grow0 : grow0 + TC_ROWS;
         for (int st = 0; st < stages_per_tile; st += 2, n += 2) {
           const int k0 = kbase + st * TC_KT;
@@ -417,7 +426,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       const uint32_t idesc = make_idesc(128, ncols);
       if (!mbar_wait_warp(acc_empty_bar, (ti & 1u) ^ 1u, abort_flag, args.status)) break;
       tc_fence_after();
-      for (int st = 0; st < stages_per_tile; ++st) {
+      for (int st = 0; st < stages_per_tile; st += HK) {
         const uint32_t ab = 8u * (2 * as + mset);
         const uint32_t sub = static_cast<uint32_t>(st) & 1u;  // half of the token slot (tiles hold an even number of stages)
         if ((sub == 0 && !mbar_wait_warp(xfull + 8u * xs, xph, abort_flag, args.status)) ||
@@ -427,16 +436,19 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         }
         tc_fence_after();
         const uint32_t b_lo = ((x_base + xs * TC_XSLOT + sub * TC_XSUB) & 0x3FFFFu) >> 4;
+        const bool last = HK == 2 || sub == 1;  // of the token slot
         if (elect_one()) {
-          tc_mma_ts_x4(acc, a_set + as * 64, b_lo, desc_hi, idesc, st > 0 ? 1u : 0u);
+          tc_mma_ts_x4(acc, a_set + as * (64 * HK), b_lo, desc_hi, idesc, st > 0 ? 1u : 0u);
+          if constexpr (HK == 2)
+            tc_mma_ts_x4(acc, a_set + as * 128 + 64, b_lo + (TC_XSUB >> 4), desc_hi, idesc, 1u);
           tc_commit(a_free + ab);
-          if (sub) tc_commit(xempty + 8u * xs);
+          if (last) tc_commit(xempty + 8u * xs);
         }
         __syncwarp();
-        if (sub) {
+        if (last) {
           if (++xs == TC_XSLOTS) { xs = 0; xph ^= 1u; }
         }
-        if (++as == TC_ASLOTS) { as = 0; aph ^= 1u; }
+        if (++as == HSLOTS) { as = 0; aph ^= 1u; }
       }
       if (ok && elect_one()) tc_commit(acc_full_bar);
       __syncwarp();
@@ -448,9 +460,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const int wq = warp & 3;                // TMEM lane quarter
     const int row = wq * 32 + lane;         // weight row within the set = TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(wq * 32) << 16;
-    const int sw = row & 7;                 // 128-byte swizzle term of this row
-    uint32_t n = 0, ti = 0;
+    uint32_t ti = 0;
     bool ok = true;
+    // ring positions of this group's next hand-over and the parities of its waits.
+    // With HK = 1 a group takes its 64-k half of every weight slot, with HK = 2 every
+    // second weight slot whole; hand-over slots alternate between the groups.
+    uint32_t ws = HK == 2 ? grp : 0, wph = 0, ss = 0, sph = 0, as = grp, aph = 1;
 
     // Drains the two accumulators of a finished tile.  Each of the four
     // (group, set) warp sets takes every fourth 16-token column chunk.
@@ -458,12 +473,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       if (!mbar_wait_warp(acc_full_bar, tix & 1u, abort_flag, args.status)) return false;
       tc_fence_after();
       if constexpr (NMAT == 2) {
-        int col = (nt & 0xffff) * TC_ROWS + row;
+        int col = (nt & 0xffff) * args.row_tile + row;
         if (args.out_kperm) col = (col & ~7) | ((col & 3) << 1) | ((col >> 2) & 1);
         __half* obase = static_cast<__half*>(args.out) + static_cast<size_t>(row0) * args.N + col;
         const size_t ostride = static_cast<size_t>(args.N);
         const bool silu = args.act == B200MOE_ACT_SILU;
         float amax = 0.f;
+        // lanes past a short row tile hold products with whatever their slot rows held:
+        // neither stored nor range-checked
+        const int lane_rows = row < args.row_tile ? rows : 0;
         for (int c0 = (grp * 2 + set) * 16; c0 < ncols; c0 += 64) {
 #pragma unroll 1
           for (int h8 = 0; h8 < 16; h8 += 8) {
@@ -472,7 +490,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             tmem_ld8(tmem + lane_addr + TC_COL_ACC1 + c0 + h8, u);
             tmem_wait_ld();
             __half* o = obase + static_cast<size_t>(c0 + h8) * ostride;
-            const int lim = rows - c0 - h8;  // token rows of the segment among these eight
+            const int lim = lane_rows - c0 - h8;  // token rows of the segment among these eight
             if (lim >= 8) {
               if (silu) {
 #pragma unroll
@@ -542,74 +560,90 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       int e, nt, row0, rows, ncols;
       decode(tile, e, nt, row0, rows, ncols);
       for (int sg = 0; sg < stages_per_tile / TC_SGROUP && ok; ++sg) {
-        const uint32_t g = n / TC_SGROUP;
-        const int ss = g % TC_SSLOTS;
-        if (!mbar_wait_warp(sfull + 8u * ss, (g / TC_SSLOTS) & 1u, abort_flag, args.status)) { ok = false; break; }
-        // Q8_0: 8 fp16 block scales of the 256-k group; Q4_K: 8 (scale, min) half2 pairs
-        uint32_t scw[8];
-        if constexpr (Q4) {
-          lds128(scale_base + ss * TC_SSLOT + set * TC_SSET + row * 32, *reinterpret_cast<uint32_t(*)[4]>(&scw[0]));
-          lds128(scale_base + ss * TC_SSLOT + set * TC_SSET + row * 32 + 16, *reinterpret_cast<uint32_t(*)[4]>(&scw[4]));
-        } else {
-          lds128(scale_base + ss * TC_SSLOT + set * TC_SSET + row * 16, *reinterpret_cast<uint32_t(*)[4]>(&scw[0]));
+        if (!mbar_wait_warp(sfull + 8u * ss, sph, abort_flag, args.status)) { ok = false; break; }
+        // scales of this group's two 64-k stages of the four: Q8_0: one word (two fp16
+        // block scales) per stage; Q4_K: two (scale, min) half2 pairs per stage
+        uint32_t scw[2][Q4 ? 2 : 1];
+        {
+          const uint32_t srow = scale_base + ss * TC_SSLOT + set * TC_SSET + row * (Q4 ? 32 : 16);
+          if constexpr (Q4) {
+            uint32_t lo[4], hi[4];
+            lds128(srow, lo);
+            lds128(srow + 16, hi);
+            if constexpr (HK == 2) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) scw[i >> 1][i & 1] = grp ? hi[i] : lo[i];
+            } else {
+              scw[0][0] = grp ? lo[2] : lo[0]; scw[0][1] = grp ? lo[3] : lo[1];
+              scw[1][0] = grp ? hi[2] : hi[0]; scw[1][1] = grp ? hi[3] : hi[1];
+            }
+          } else {
+            uint32_t q[4];
+            lds128(srow, q);
+            scw[0][0] = grp ? q[HK] : q[0];
+            scw[1][0] = grp ? q[3] : q[3 - HK];
+          }
         }
         fence_proxy_async_smem();  // reads done before TMA may refill the slot
         __syncwarp();
         if (lane == 0) mbar_arrive(sempty + 8u * ss);
+        if (++ss == TC_SSLOTS) { ss = 0; sph ^= 1u; }
 #pragma unroll
-        for (int s4 = 0; s4 < 4; ++s4, ++n) {
-          if ((s4 & 1) != grp) continue;
-          // this group's half (64 k) of the weight slot
-          const uint32_t wi = n >> 1;
-          const int ws = wi % TC_WSLOTS;
-          const int as = n % TC_ASLOTS;  // even slot count: slot parity == this group's stage parity
-          if (!mbar_wait_warp(wfull + 8u * ws, (wi / TC_WSLOTS) & 1u, abort_flag, args.status)) { ok = false; break; }
-          uint32_t v[32];
-          if constexpr (Q4) {
-            // 64-byte rows (128 k of nibbles), 64-byte swizzle; this stage = chunks 2*grp, 2*grp+1
-            const uint32_t wrow = smem_base + ws * TC_WSLOT + set * TC_WSET + row * 64;
-            const int sw64 = (row >> 1) & 3;
-            uint32_t q[2][4];
+        for (int h = 0; h < 2 / HK; ++h) {
+          if (!mbar_wait_warp(wfull + 8u * ws, wph, abort_flag, args.status)) { ok = false; break; }
+          // this group's 64-byte (Q4_K 32-byte) pieces of its row in the slot
+          constexpr int CH = Q4 ? 2 : 4;  // 16-byte chunks per 64-k stage
+          const uint32_t wrow = smem_base + ws * TC_WSLOT + set * TC_WSET + row * (Q4 ? 64 : 128);
+          const int swz = Q4 ? (row >> 1) & 3 : row & 7;
+          uint32_t q[HK][CH][4];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) lds128(wrow + (((2 * grp + c) ^ sw64) << 4), q[c]);
-            fence_proxy_async_smem();  // reads done before TMA may refill the slot
-            __syncwarp();
-            if (lane == 0) mbar_arrive(wempty + 8u * ws);
+          for (int j = 0; j < HK; ++j)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const uint32_t sm = scw[2 * s4 + c];  // sub-block (32 k) scale / min
-              const __half2 ds = u32_as_h2(__byte_perm(sm, sm, 0x1010));
-              const __half2 dm = u32_as_h2(__byte_perm(sm, sm, 0x3232));
+            for (int c = 0; c < CH; ++c)
+              lds128(wrow + ((((HK == 2 ? j : grp) * CH + c) ^ swz) << 4), q[j][c]);
+          fence_proxy_async_smem();  // reads done before TMA may refill the slot
+          __syncwarp();
+          if (lane == 0) mbar_arrive(wempty + 8u * ws);
+          ws += HK;
+          if (ws >= TC_WSLOTS) { ws -= TC_WSLOTS; wph ^= 1u; }
 #pragma unroll
-              for (int j = 0; j < 4; ++j)
-                dequant_q4x8(q[c][j], ds, dm, *reinterpret_cast<uint32_t(*)[4]>(&v[c * 16 + j * 4]));
+          for (int j = 0; j < HK; ++j) {
+            uint32_t v[32];
+            const uint32_t(&sc)[Q4 ? 2 : 1] = scw[HK == 2 ? j : h];
+            if constexpr (Q4) {
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                const __half2 ds = u32_as_h2(__byte_perm(sc[c], sc[c], 0x1010));
+                const __half2 dm = u32_as_h2(__byte_perm(sc[c], sc[c], 0x3232));
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  dequant_q4x8(q[j][c][i], ds, dm, *reinterpret_cast<uint32_t(*)[4]>(&v[c * 16 + i * 4]));
+              }
+            } else {
+              const __half2 s_lo = u32_as_h2(__byte_perm(sc[0], sc[0], 0x1010));
+              const __half2 s_hi = u32_as_h2(__byte_perm(sc[0], sc[0], 0x3232));
+#pragma unroll
+              for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  dequant_q8x4(q[j][c][i], c < 2 ? s_lo : s_hi, v[c * 8 + 2 * i], v[c * 8 + 2 * i + 1]);
             }
-          } else {
-            const uint32_t wrow = smem_base + ws * TC_WSLOT + set * TC_WSET + row * 128;
-            uint32_t q[4][4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) lds128(wrow + (((4 * grp + c) ^ sw) << 4), q[c]);
-            fence_proxy_async_smem();  // reads done before TMA may refill the slot
-            __syncwarp();
-            if (lane == 0) mbar_arrive(wempty + 8u * ws);
-            const __half2 s_lo = u32_as_h2(__byte_perm(scw[s4], scw[s4], 0x1010));
-            const __half2 s_hi = u32_as_h2(__byte_perm(scw[s4], scw[s4], 0x3232));
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                dequant_q8x4(q[c][j], c < 2 ? s_lo : s_hi, v[c * 8 + 2 * j], v[c * 8 + 2 * j + 1]);
+            if (j == 0) {
+              if (!mbar_wait_warp(a_free + 8u * (2 * as + set), aph, abort_flag, args.status)) { ok = false; break; }
+              tc_fence_after();
+            }
+            tmem_st32(tmem + lane_addr + TC_COL_A + (as * HK + j) * 64 + set * 32, v);
           }
-          if (!mbar_wait_warp(a_free + 8u * (2 * as + set), ((n / TC_ASLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
-          tc_fence_after();
-          tmem_st32(tmem + lane_addr + TC_COL_A + as * 64 + set * 32, v);
+          if (!ok) break;
           tmem_wait_st();
           tc_fence_before();
           // one arrival per warp: 256 arrivals per stage on one barrier word
           // serialise in shared memory
           __syncwarp();
           if (lane == 0) mbar_arrive(a_ready + 8u * (2 * as + set));
-          if (s4 < 2 && sg == 0 && have_prev) {
+          as += 2;
+          if (as >= HSLOTS) { as -= HSLOTS; aph ^= 1u; }
+          if (h == 0 && sg == 0 && have_prev) {
             have_prev = false;
             if (!epilogue(p_nt, p_row0, p_rows, p_ncols, p_ti)) { ok = false; break; }
           }
@@ -667,6 +701,38 @@ int tc_pick_tok_tile(int tok_tile, int pairs, int experts) {
   return tok_tile;
 }
 
+// Expected token tiles over all experts when `pairs` rows fall on them evenly:
+// the row count of one expert is taken as normal with the mean's variance, and
+// its tiles are 1 + the number of tile boundaries it is expected to pass.
+double tc_expected_token_tiles(int pairs, int experts, int tok_tile) {
+  const double mean = static_cast<double>(pairs) / (experts > 0 ? experts : 1);
+  const double sd = mean > 1.0 ? sqrt(mean) : 1.0;
+  double tiles = 1.0;
+  for (int b = tok_tile; b < mean + 4.0 * sd; b += tok_tile)
+    tiles += 0.5 * erfc((b + 0.5 - mean) / (1.4142135623730951 * sd));
+  return tiles * (pairs < experts ? pairs : experts);
+}
+
+// Rows of each weight set per gate/up tile.  The narrow token tiles stream their
+// weights, so a tile's time is its rows' (+ about 8 rows' worth at the boundary)
+// and what counts is the last wave of SMs: of the heights that divide the matrix
+// take the one with the least rows over all waves.  Eight experts of 14336 rows: 896
+// tiles of 128 rows are 7 waves for 6.05 waves of work, 1024 tiles of 112 rows 6.92.
+// The 192-token variant is bound by its MMAs, which always work on 128 rows.
+int tc_row_tile(int rows, double token_tiles, int tok_tile) {
+  if (tok_tile > 128) return TC_ROWS;
+  const int sms = sm_count();
+  int best = TC_ROWS;
+  double best_cost = 0.0;
+  for (int r = TC_ROWS; r >= 64; r -= 16) {
+    if (rows % r != 0) continue;
+    const double waves = ceil(token_tiles * (rows / r) / sms);
+    const double cost = waves * (r + 8);
+    if (r == TC_ROWS || cost < 0.98 * best_cost) { best_cost = cost; best = r; }
+  }
+  return best;
+}
+
 // Token-tile tensor maps with box heights 16, 32, 64, 96, 128 and 192 (maps[4..9]).
 int tc_token_maps(CUtensorMap* maps, const void* x, int pairs, uint64_t row_bytes) {
   const int heights[6] = {16, 32, 64, 96, 128, 192};
@@ -688,17 +754,17 @@ int tc_check(const b200moe_weight_t* w, const char* name) {
   return B200MOE_OK;
 }
 
-int tc_weight_map(const b200moe_weight_t* w, CUtensorMap* tw, CUtensorMap* ts) {
-  // 128-byte wide boxes of int8 with the 128-byte swizzle: 128 rows x 128 k;
-  // scale boxes of 8 fp16 (256 k) x 128 rows, unswizzled
+int tc_weight_map(const b200moe_weight_t* w, CUtensorMap* tw, CUtensorMap* ts, int box_rows = TC_ROWS) {
+  // 128-byte wide boxes of int8 with the 128-byte swizzle: box_rows x 128 k;
+  // scale boxes of 8 fp16 (256 k) x box_rows, unswizzled
   const uint64_t rows = static_cast<uint64_t>(w->experts) * w->rows;
   if (w->layout == B200MOE_LAYOUT_Q4_K) {
     // nibbles: 64-byte wide boxes (128 k), 64-byte swizzle; (scale, min) pairs: 32 bytes per row
-    if (int rc = make_tmap_2d_sw(tw, w->qs, rows, w->cols / 2, TC_ROWS, 64, 64)) return rc;
-    return make_tmap_2d_sw(ts, w->sub, rows, static_cast<uint64_t>(w->cols) / 32 * 4, TC_ROWS, 32, 0);
+    if (int rc = make_tmap_2d_sw(tw, w->qs, rows, w->cols / 2, box_rows, 64, 64)) return rc;
+    return make_tmap_2d_sw(ts, w->sub, rows, static_cast<uint64_t>(w->cols) / 32 * 4, box_rows, 32, 0);
   }
-  if (int rc = make_tmap_2d_sw(tw, w->qs, rows, w->cols, TC_ROWS, 128, 128)) return rc;
-  return make_tmap_2d_sw(ts, w->d, rows, static_cast<uint64_t>(w->cols) / 32 * 2, TC_ROWS, 16, 0);
+  if (int rc = make_tmap_2d_sw(tw, w->qs, rows, w->cols, box_rows, 128, 128)) return rc;
+  return make_tmap_2d_sw(ts, w->d, rows, static_cast<uint64_t>(w->cols) / 32 * 2, box_rows, 16, 0);
 }
 
 }  // namespace
@@ -723,13 +789,15 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
                "tensor kernel: gate and up shapes or layouts differ");
   B200_REQUIRE(gate->rows % TC_ROWS == 0, "tensor kernel: ffn (%d) must be a multiple of 128", gate->rows);
   if (pairs == 0) return B200MOE_OK;
-  CUtensorMap maps[10];
-  if (int rc = tc_weight_map(gate, &maps[0], &maps[2])) return rc;
-  if (int rc = tc_weight_map(up, &maps[1], &maps[3])) return rc;
-  if (int rc = tc_token_maps(maps, xs, pairs, static_cast<uint64_t>(gate->cols) * 2)) return rc;
   TcArgs a{};
+  a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, gate->experts);
+  a.row_tile = tc_row_tile(gate->rows, tc_expected_token_tiles(pairs, gate->experts, a.tok_tile), a.tok_tile);
+  CUtensorMap maps[10];
+  if (int rc = tc_weight_map(gate, &maps[0], &maps[2], a.row_tile)) return rc;
+  if (int rc = tc_weight_map(up, &maps[1], &maps[3], a.row_tile)) return rc;
+  if (int rc = tc_token_maps(maps, xs, pairs, static_cast<uint64_t>(gate->cols) * 2)) return rc;
   a.seg = seg; a.E = gate->experts; a.N = gate->rows; a.K = gate->cols;
-  a.ntiles = gate->rows / TC_ROWS; a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, gate->experts); a.P = pairs; a.act = act;
+  a.ntiles = gate->rows / a.row_tile; a.P = pairs; a.act = act;
   a.ksplit = 1;
   a.out_kperm = out_kperm;
   a.out = a_out; a.status = device_status_ptr();
@@ -744,23 +812,23 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
 }
 
 int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs) {
-  // Few tiles (expert-parallel ranks with one or two experts) leave SMs idle:
-  // split the long reduction into up to four partitions when that fills the
-  // waves better.  est_pairs is the expected number of rows, not a bound.
+  // The long reduction is split into up to eight partitions when that fills the
+  // waves of SMs better.  Cost in 64-k stages (about 0.4 us each): waves of items,
+  // each its stages and about 3 for the boundary, plus writing and reading back the
+  // partial sums at the copy bandwidth.  est_pairs is the expected number of rows,
+  // not a bound; the number of token tiles is its expectation (195 rows per expert
+  // are 1.5 tiles of 192, not 2).
   const int stages = down->cols / TC_KT;
   const int sms = sm_count();
-  const int per_expert = est_pairs / (down->experts > 0 ? down->experts : 1);
-  const long long tiles = static_cast<long long>(down->experts) * (down->rows / (2 * TC_ROWS)) *
-                          ((per_expert + 191) / 192 > 0 ? (per_expert + 191) / 192 : 1);
-  if (tiles >= 2ll * sms) return 1;
+  const int tok = tc_pick_tok_tile(TC_NTOK, est_pairs, down->experts);
+  const double tiles = tc_expected_token_tiles(est_pairs, down->experts, tok) * (down->rows / (2 * TC_ROWS));
+  const double part = static_cast<double>(est_pairs) * down->rows * 8.0 / 6.5e6 / 0.4;
   int best = 1;
-  double best_eff = 0.0;
-  for (int ks = 1; ks <= 4; ks *= 2) {
+  double best_cost = 0.0;
+  for (int ks = 1; ks <= 8; ks *= 2) {
     if (stages % (4 * ks) != 0) break;
-    const long long items = tiles * ks;
-    const long long waves = (items + sms - 1) / sms;
-    const double eff = static_cast<double>(items) / (waves * sms) - 0.03 * (ks - 1);
-    if (eff > best_eff) { best_eff = eff; best = ks; }
+    const double cost = ceil(tiles * ks / sms) * (stages / ks + 3) + ks * part;
+    if (ks == 1 || cost < 0.98 * best_cost) { best_cost = cost; best = ks; }
   }
   return best;
 }
@@ -780,6 +848,7 @@ int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile
   a.seg = seg; a.E = down->experts; a.N = down->rows; a.K = down->cols;
   B200_REQUIRE(ksplit >= 1 && (down->cols / TC_KT) % (4 * ksplit) == 0, "tensor kernel: bad k split %d",
                ksplit);
+  a.row_tile = TC_ROWS;
   a.ntiles = down->rows / (2 * TC_ROWS); a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, down->experts); a.P = pairs; a.act = 0;
   a.ksplit = ksplit;
   a.out = d_out; a.status = device_status_ptr();

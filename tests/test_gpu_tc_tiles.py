@@ -1,0 +1,43 @@
+"""Tiles of the tensor kernel that only some sizes reach: row tiles shorter than 128
+(narrow token tiles, where they fill the SMs better), two-stage hand-overs and k
+splits, on ragged segments, against the streaming kernel and the oracle."""
+import pytest
+import torch
+
+from oracle import moe_oracle as orc
+from shark_platform_b200 import synthetic as syn
+from helpers import b200_block, device_input, oracle_params
+
+pytestmark = pytest.mark.gpu
+
+
+# ffn 1792 = 16 x 112 = 14 x 128, 768 = 12 x 64 = 8 x 96 = 6 x 128, 1280 = 10 x 128 = 20 x 64
+@pytest.mark.parametrize("kind", [syn.Q8_0, syn.Q4_K])
+@pytest.mark.parametrize("ffn,activation", [(1792, "silu"), (768, "gelu"), (1280, "silu")])
+@pytest.mark.parametrize("tokens", [1, 17, 129, 400])
+def test_short_row_tiles_match_the_oracle(kind, ffn, activation, tokens):
+    from shark_platform_b200 import moe
+
+    spec = syn.CaseSpec("tiles", tokens, 512, ffn, kind=kind, activation=activation, router_bias="zipf",
+                        norm_weight="perturbed", seed=71)
+    case = syn.make_case(spec)
+    h = device_input(case)
+    got = b200_block(case, regime="tensor")(h)
+    again = b200_block(case, regime="tensor")(h)
+    assert torch.equal(got, again), "two runs differ: a race"
+    stream = b200_block(case, regime="stream")(h)
+    assert moe.device_status() == 0
+    assert orc.rel_l2(got.float().cpu(), stream.float().cpu()) < 5e-3  # both rounded to bf16
+    want, _ = orc.moe_block(case.h, oracle_params(case), form="per_expert")
+    assert orc.rel_l2(got.float().cpu(), want) < 2e-2
+
+
+def test_fewer_tokens_after_more_still_fit_the_workspace():
+    """The k split, and with it the bytes per row, is larger at some smaller token counts."""
+    spec = syn.CaseSpec("shrink", 1100, 512, 512, kind=syn.Q8_0, seed=72)
+    case = syn.make_case(spec)
+    h = device_input(case)
+    blk = b200_block(case)
+    for n in (1100, 512, 100, 3, 1):
+        want = b200_block(case)(h[:n] if h.dim() == 2 else h.reshape(-1, 512)[:n])
+        assert torch.equal(blk(h.reshape(-1, 512)[:n]), want)
