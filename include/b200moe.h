@@ -187,6 +187,21 @@ int b200moe_gate_up(const void* xs, const int32_t* seg_offsets, int32_t pairs,
 int b200moe_down_ksplit(const b200moe_weight_t* down, int32_t pairs, int32_t max_segment,
                         int regime);
 
+/* Dense quantised linears that share their input: outs[i] = x weights[i]^T for
+ * count (1..4) stacks of one matrix each (Q8_0 or Q4_K, equal cols, a multiple of
+ * 256; rows multiples of 128) — sharktank's ops.linear / ops.matmul on such weights
+ * (ops/qlinear_impls.py:158-172, ops/custom_impls.py:66-128).  x: [rows, cols] fp32,
+ * fp16 or bf16, rounded to fp16 for the products; with norm_weight (fp32 [cols]) the
+ * row is RMS-normalised first (layers/norm.py:34-41).  outs[i]: [rows, weights[i]->rows]
+ * of out_dtype; residual (NULL or out_dtype, the shape of outs[0]) is added to the
+ * rounded outs[0].  x, norm_weight, residual and outs 16-byte aligned.  Workspace of
+ * b200moe_linear_workspace_bytes(...) bytes (0 for bad arguments or no rows). */
+size_t b200moe_linear_workspace_bytes(const b200moe_weight_t* const* weights, int32_t count, int32_t rows,
+                                      int x_dtype, int has_norm);
+int b200moe_linear(const void* x, int x_dtype, int32_t rows, const float* norm_weight, float eps,
+                   const b200moe_weight_t* const* weights, int32_t count, void* const* outs, int out_dtype,
+                   const void* residual, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Down projection per expert segment: the "mek,menk->men" einsum
  * (layers/ffn_moe_block.py:70-72; ops/default_impls.py:84-94).  a fp16
  * [pairs,F]; d_out fp32 [ksplit, pairs, d] partial sums with ksplit =

@@ -97,6 +97,7 @@ lib = ctypes.CDLL(LIB_PATH)
 _W = POINTER(WeightDesc)
 _L = POINTER(LayerDesc)
 _P = c_void_p
+WeightPtr = _W
 
 _PROTOS = {
     "b200moe_version": (c_char_p, []),
@@ -117,6 +118,9 @@ _PROTOS = {
     "b200moe_gate_up": (c_int, [_P, _P, c_int32, c_int32, _W, _W, c_int, c_int, c_int32, _P, _P]),
     "b200moe_down_ksplit": (c_int, [_W, c_int32, c_int32, c_int]),
     "b200moe_down": (c_int, [_P, _P, c_int32, c_int32, _W, c_int, c_int32, _P, _P]),
+    "b200moe_linear_workspace_bytes": (c_size_t, [POINTER(_W), c_int32, c_int32, c_int, c_int]),
+    "b200moe_linear": (c_int, [_P, c_int, c_int32, _P, c_float, POINTER(_W), c_int32, POINTER(_P), c_int, _P, _P,
+                               c_size_t, _P]),
     "b200moe_down_noalloc": (c_int, [_P, _P, c_int32, c_int32, _W, _P, _P]),
     "b200moe_combine": (c_int, [_P, c_int, c_int32, c_int32, _P, _P, _P, c_int, c_int32, _L, c_int, _P, c_int, _P]),
     "b200moe_exchange_plan": (c_int, [_P, c_int32, c_int32, _P, _P, _P, _P]),

@@ -104,7 +104,7 @@ class B200PagedAttentionBlock(torch.nn.Module):
         if cache.attn_head_count != head_count_kv or cache.attn_head_dim != head_dim:
             raise C.B200MoeError("the cache's heads / head_dim differ from the block's")
         w = lambda name: theta(name).tensor("weight")
-        self._norm_w = _moe._unbox(w("attn_norm")).to(torch.float32).contiguous()
+        self._norm_w = _moe._aligned(_moe._unbox(w("attn_norm")).to(torch.float32))
         _moe._require_cuda(self._norm_w, "attn_norm.weight")
         self._out_norm_w = None
         if theta.optional_tensor("attn_output_norm") is not None:
@@ -129,6 +129,12 @@ class B200PagedAttentionBlock(torch.nn.Module):
             return y
         wt = _moe._unbox(weight) if not isinstance(weight, torch.Tensor) else weight
         return F.linear(x, wt.to(x.dtype), None if bias is None else _moe._unbox(bias).to(x.dtype))
+
+    @staticmethod
+    def _fits_linear(*weights) -> bool:
+        """Every weight is one that `moe.matmul_quantized` takes."""
+        return all(_is_quantized(w) and len(w.shape) == 2 and int(w.shape[0]) % 256 == 0 and
+                   int(w.shape[1]) % 256 == 0 for w in weights)
 
     def _norm(self, x, weight):
         y = torch.empty_like(x)
@@ -172,12 +178,23 @@ class B200PagedAttentionBlock(torch.nn.Module):
         decode = start_positions is not None
         if decode and sl != 1:
             raise C.B200MoeError("a decode step brings one token per sequence")
-        x = self._norm(h.contiguous(), self._norm_w)
+        hc = h.contiguous()
+        # the output projection with the residual, in one call
+        fused_out = (self._fits_linear(self._wo) and [int(n) for n in self._wo.shape] == [d, H * hd] and
+                     self._bias["attn_output"] is None and self._out_norm_w is None)
         if self._wqkv is not None:
+            x = self._norm(hc, self._norm_w)
             qkv = F.linear(x, self._wqkv.to(x.dtype))
             q, k, v = torch.split(qkv, [H * hd, Hkv * hd, Hkv * hd], dim=-1)
             q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        elif self._fits_linear(self._wq, self._wk, self._wv) and int(self._wq.shape[1]) == d:
+            # norm and the three projections in one call
+            q, k, v = _moe.linear_rows(hc.view(bs * sl, d), [_moe.prepare_linear(w) for w in (self._wq, self._wk, self._wv)],
+                                       norm_weight=self._norm_w, eps=float(self.rms_epsilon))
+            q, k, v = (y if bias is None else y + _moe._unbox(bias).to(y.dtype) for y, bias in
+                       zip((q, k, v), (self._bias[n] for n in ("attn_q", "attn_k", "attn_v"))))
         else:
+            x = self._norm(hc, self._norm_w)
             q = self._linear(x, self._wq, self._bias["attn_q"]).contiguous()
             k = self._linear(x, self._wk, self._bias["attn_k"]).contiguous()
             v = self._linear(x, self._wv, self._bias["attn_v"]).contiguous()
@@ -190,9 +207,8 @@ class B200PagedAttentionBlock(torch.nn.Module):
             positions = (torch.arange(sl, device=dev, dtype=torch.int32) + int(start_index)).repeat(bs)
         page_ids = seq_block_ids.to(torch.int32).contiguous()
         self._desc.page_count = slab.shape[0]
-        k_out = v_out = None
-        if not decode:
-            k_out, v_out = torch.empty_like(k), torch.empty_like(v)
+        # prefill attends the fresh K and V: K is rotated in place, V is used as it is
+        k_out, v_out = (None, None) if decode else (k, v)
         with torch.cuda.device(dev):
             C.check(C.lib.b200moe_attn_rope_kv_write(
                 _p(q), _p(k), _p(v), _p(k_out), _p(v_out), _DT[q.dtype], _p(slab), _DT[slab.dtype],
@@ -205,7 +221,9 @@ class B200PagedAttentionBlock(torch.nn.Module):
             # reference's decode mask leaves unmasked)
             seq_lens = (positions + 1).contiguous()
             max_len = page_ids.shape[1] * stride
-            out = torch.empty(bs, H * hd, dtype=h.dtype, device=dev)
+            # a Q8_0 output projection reads fp16 rows: no cast in between
+            direct = fused_out and _moe._layout_name(self._wo) == "BlockScaledLayout"
+            out = torch.empty(bs, H * hd, dtype=torch.float16 if direct else h.dtype, device=dev)
             nbytes = C.lib.b200moe_attn_decode_scratch_bytes(ctypes.byref(self._desc), bs, H, max_len)
             if self._scratch is None or self._scratch.numel() < nbytes or self._scratch.device != dev:
                 self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
@@ -218,8 +236,8 @@ class B200PagedAttentionBlock(torch.nn.Module):
             attn = out.view(bs, 1, H * hd)
         else:
             qh = q.view(bs, sl, H, hd).transpose(1, 2)
-            kh = k_out.view(bs, sl, Hkv, hd).transpose(1, 2)
-            vh = v_out.view(bs, sl, Hkv, hd).transpose(1, 2)
+            kh = k.view(bs, sl, Hkv, hd).transpose(1, 2)
+            vh = v.view(bs, sl, Hkv, hd).transpose(1, 2)
             mask = None if attention_mask is None else attention_mask.to(q.dtype)
             if self.softcap is None:
                 attn = F.scaled_dot_product_attention(qh, kh, vh, attn_mask=mask, is_causal=mask is None,
@@ -235,6 +253,10 @@ class B200PagedAttentionBlock(torch.nn.Module):
                     w = w + torch.full((sl, sl), float("-inf"), device=dev, dtype=w.dtype).triu(1)
                 attn = torch.matmul(torch.softmax(w.float(), dim=-1).to(qh.dtype), vh)
             attn = attn.transpose(1, 2).reshape(bs, sl, H * hd)
+        if fused_out:
+            y, = _moe.linear_rows(attn.reshape(bs * sl, H * hd), [_moe.prepare_linear(self._wo)],
+                                  residual=hc.view(bs * sl, d), out_dtype=h.dtype)
+            return y.view(bs, sl, d)
         y = self._linear(attn, self._wo, self._bias["attn_output"])
         if self._out_norm_w is not None:
             y = self._norm(y.contiguous(), self._out_norm_w)

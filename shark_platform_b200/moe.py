@@ -630,27 +630,62 @@ def matmul_quantized(lhs, rhs, *, transpose_rhs: bool = False):
     if k % 256 != 0 or n % 256 != 0 or x.shape[-1] != k:
         return NotImplemented
 
-    class _AsExperts:  # the same planes seen as a stack of one expert
-        pass
+    x2 = x.reshape(-1, k)
+    if x.dtype not in _DT:
+        x2 = x2.to(torch.float16)
+    out, = linear_rows(x2, [prepare_linear(rhs)], out_dtype=x.dtype if x.dtype in _DT else torch.float32)
+    return out.view(*x.shape[:-1], n).to(x.dtype)
 
+
+class _AsExperts:
+    """A [N, K] weight's planes seen as a stack of one expert."""
+
+    def __init__(self, rhs):
+        self.layout_type = rhs.layout_type
+        self.shape = [1] + [int(v) for v in rhs.shape]
+        self.unpack = rhs.unpack
+
+
+def prepare_linear(rhs) -> PreparedWeight:
+    """`prepare_weight` for a [N, K] planar weight; kept on the tensor object."""
     holder = getattr(rhs, "_b200moe_as_experts", None)
     if holder is None:
-        holder = _AsExperts()
-        holder.layout_type = rhs.layout_type
-        holder.shape = [1, n, k]
-        holder.unpack = rhs.unpack
+        holder = _AsExperts(rhs)
         try:
             rhs._b200moe_as_experts = holder
         except AttributeError:
             pass
-    w = prepare_weight(holder)
-    rows = x.reshape(-1, k).to(torch.float16).contiguous()
-    m = rows.shape[0]
-    if C.lib.b200moe_kperm(w.layout, C.REGIME_AUTO, m):
-        rows = rows.view(m, -1, 2, 4).transpose(2, 3).reshape(m, -1).contiguous()
-    seg = torch.tensor([0, m], dtype=torch.int32, device=x.device)
-    out = grouped_matmul(rows, seg, w, max(m, 1))
-    return out.view(*x.shape[:-1], n).to(x.dtype)
+    return prepare_weight(holder)
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary (a view into a larger buffer may not be)."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
+def linear_rows(x: torch.Tensor, weights, *, norm_weight: Optional[torch.Tensor] = None, eps: float = 0.0,
+                residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None):
+    """[x W^T for W in weights] for fp32 / fp16 / bf16 rows x [m, K] and prepared
+    [N, K] weights: one library call (`b200moe_linear`).  `norm_weight`: RMS-normalise
+    the rows first; `residual` (of the output type) is added to the first output."""
+    x = _aligned(x)
+    m, dev = x.shape[0], x.device
+    out_dtype = x.dtype if out_dtype is None else out_dtype
+    outs = [torch.empty(m, w.rows, dtype=out_dtype, device=dev) for w in weights]
+    if m == 0:
+        return outs
+    n = len(weights)
+    wp = (C.WeightPtr * n)(*[ctypes.pointer(w.desc) for w in weights])
+    op = (ctypes.c_void_p * n)(*[o.data_ptr() for o in outs])
+    if residual is not None:
+        residual = _aligned(residual)
+    with torch.cuda.device(dev):
+        nbytes = C.lib.b200moe_linear_workspace_bytes(wp, n, m, _DT[x.dtype], norm_weight is not None)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        C.check(C.lib.b200moe_linear(_ptr(x), _DT[x.dtype], m, _ptr(norm_weight), eps, wp, n, op, _DT[out_dtype],
+                                     _ptr(residual), _ptr(ws), nbytes, _stream()), "linear")
+    return outs
 
 
 def linear_quantized(input, weight, bias=None, *, accum_dtype=None):
