@@ -188,7 +188,7 @@ int b200moe_down_ksplit(const b200moe_weight_t* down, int32_t pairs, int32_t max
                         int regime);
 
 /* Dense quantised linears that share their input: outs[i] = x weights[i]^T for
- * count (1..4) stacks of one matrix each (Q8_0 or Q4_K, equal cols, a multiple of
+ * count (1..3) stacks of one matrix each (Q8_0 or Q4_K, equal cols, a multiple of
  * 256; rows multiples of 128) — sharktank's ops.linear / ops.matmul on such weights
  * (ops/qlinear_impls.py:158-172, ops/custom_impls.py:66-128).  x: [rows, cols] fp32,
  * fp16 or bf16, rounded to fp16 for the products; with norm_weight (fp32 [cols]) the

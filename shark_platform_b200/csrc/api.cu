@@ -126,9 +126,15 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // Upper bound of the tensor kernels' token tile (b200moe_set_token_tile).
 int g_token_tile = 192;
 
-// Above this many tokens the tensor-memory kernel takes over from the
-// weight-streaming kernel (where the layout allows it).
-constexpr int TENSOR_MIN_TOKENS = 97;
+// From this many tokens the tensor-memory kernel takes over from the
+// weight-streaming kernel (where the layout allows it).  One B200, Mixtral layer, us
+// per call, stream / tensor: Q8_0 16 tokens 278 / 292, 24 tokens 285 / 294, 32 tokens
+// 305 / 294, 64 tokens 366 / 309; Q4_K 16 tokens 261 / 267, 24 tokens 270 / 267,
+// 32 tokens 295 / 270.  A single matrix (attention projections): 4096 x 4096 Q8_0 24
+// rows 10.3 / 10.4, 32 rows 11.2 / 10.6, 64 rows 14.5 / 12.4.
+constexpr int TENSOR_MIN_TOKENS = 32;
+
+}  // namespace
 
 // `down` says which of the two products the weight belongs to (their tile
 // shapes differ).  An explicit regime is taken as given and fails in the
@@ -141,6 +147,8 @@ int pick_regime(int regime, const b200moe_weight_t* w, int max_segment, bool dow
   return (can_tensor && max_segment >= TENSOR_MIN_TOKENS) ? B200MOE_REGIME_TENSOR
                                                           : B200MOE_REGIME_STREAM;
 }
+
+namespace {
 
 // Workspace carve-up of one layer call.
 struct Workspace {

@@ -41,6 +41,9 @@ int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max
                           int out_kperm, void* a_out, cudaStream_t st);
 int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_segment,
                        const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st);
+int stream_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows);
+int launch_stream_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
+                         int ksplit, float* const* outs, cudaStream_t st);
 // -1 = wide geometry (16 consumer warps) by layout, 0 = never, 1 = always
 void set_stream_wide(int mode);
 
@@ -52,6 +55,13 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
 int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs);
 int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile,
                    const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st);
+
+int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows);
+int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
+                     int ksplit, float* const* outs, cudaStream_t st);
+
+// the kernel AUTO takes for a product of `max_segment` rows at most (api.cu)
+int pick_regime(int regime, const b200moe_weight_t* w, int max_segment, bool down);
 
 // prefill regime on CTA pairs (tc_pair_gemm.cu)
 bool tc_pair_supported_gate_up(const b200moe_weight_t* gate);

@@ -1,8 +1,8 @@
-// Quantised dense linears: y_i = x W_i^T for up to four planar Q8_0 / Q4_K weights
+// Quantised dense linears: y_i = x W_i^T for up to three planar Q8_0 / Q4_K weights
 // that share the input (the q, k and v projections), as one C call:
 //   1. linear_rows_kernel: the input rows as fp16 (optionally RMS-normalised first),
 //      in the column order(s) the weights' layouts read, plus the segment [0, rows];
-//   2. one grouped product per weight (a stack of one expert, regime by the row count);
+//   2. one launch for all weights of a layout (regime by the row count);
 //   3. linear_finish_kernel: the k-split partial sums of all outputs added, rounded
 //      to the output type and, for a block's last projection, added to the residual.
 // Replaces, per linear, a cast, a column shuffle, a torch.tensor upload of the segment
@@ -14,7 +14,7 @@
 namespace b200moe {
 namespace {
 
-constexpr int LIN_MAX = 4;
+constexpr int LIN_MAX = 3;
 constexpr int LR_THREADS = 256;
 constexpr int LR_MAXV = 4;  // 8-element vectors per thread kept in registers between the passes
 
@@ -195,6 +195,29 @@ __global__ void __launch_bounds__(256) linear_finish_kernel(const LinFinishArgs 
 
 inline size_t up1k(size_t v) { return (v + 1023) / 1024 * 1024; }
 
+// Weights of one layout go into one launch, with one kernel choice and k split.
+struct LinGroup {
+  const b200moe_weight_t* w[LIN_MAX];
+  int index[LIN_MAX];  // place in the caller's list
+  int count, ks;
+  bool tensor;
+};
+
+LinGroup lin_group(const b200moe_weight_t* const* w, int count, int rows, int layout) {
+  LinGroup g{};
+  g.tensor = true;
+  for (int i = 0; i < count; ++i) {
+    if (w[i]->layout != layout) continue;
+    g.w[g.count] = w[i];
+    g.index[g.count++] = i;
+    g.tensor = g.tensor && pick_regime(B200MOE_REGIME_AUTO, w[i], rows, true) == B200MOE_REGIME_TENSOR;
+  }
+  if (g.count > 0) g.ks = g.tensor ? tc_linear_ksplit(g.w, g.count, rows) : stream_linear_ksplit(g.w, g.count, rows);
+  return g;
+}
+
+constexpr int LIN_LAYOUTS[2] = {B200MOE_LAYOUT_Q8_0, B200MOE_LAYOUT_Q4_K};
+
 struct LinWorkspace {
   int32_t* seg;
   __half* plain;
@@ -222,10 +245,12 @@ LinWorkspace lin_carve(const b200moe_weight_t* const* w, int count, int rows, bo
   o.seg = static_cast<int32_t*>(take(8));
   if (plain && !x_ready) o.plain = static_cast<__half*>(take(row_bytes));
   if (perm) o.perm = static_cast<__half*>(take(row_bytes));
-  for (int i = 0; i < count; ++i) {
-    o.ks[i] = b200moe_down_ksplit(w[i], rows, rows, B200MOE_REGIME_AUTO);
-    o.part[i] = static_cast<float*>(take(static_cast<size_t>(o.ks[i]) * rows * w[i]->rows * 4));
+  for (int layout : LIN_LAYOUTS) {
+    const LinGroup g = lin_group(w, count, rows, layout);
+    for (int i = 0; i < g.count; ++i) o.ks[g.index[i]] = g.ks;
   }
+  for (int i = 0; i < count; ++i)
+    o.part[i] = static_cast<float*>(take(static_cast<size_t>(o.ks[i]) * rows * w[i]->rows * 4));
   o.bytes = off;
   return o;
 }
@@ -288,12 +313,19 @@ int b200moe_linear(const void* x, int x_dtype, int32_t rows, const float* norm_w
   B200_CHECK_CUDA(cudaGetLastError());
   LinFinishArgs fa{};
   long long run = 0;
-  for (int i = 0; i < count; ++i) {
-    const void* xs = b200moe_kperm(weights[i]->layout, B200MOE_REGIME_AUTO, rows) ? static_cast<const void*>(w.perm)
-                     : x_ready                                                      ? x
-                                                                                    : static_cast<const void*>(w.plain);
-    if (int rc = b200moe_down(xs, w.seg, rows, rows, weights[i], B200MOE_REGIME_AUTO, w.ks[i], w.part[i], stream))
+  for (int layout : LIN_LAYOUTS) {
+    const LinGroup g = lin_group(weights, count, rows, layout);
+    if (g.count == 0) continue;
+    const void* xs = b200moe_kperm(layout, B200MOE_REGIME_AUTO, rows) ? static_cast<const void*>(w.perm)
+                     : x_ready                                        ? x
+                                                                      : static_cast<const void*>(w.plain);
+    float* parts[LIN_MAX] = {};
+    for (int i = 0; i < g.count; ++i) parts[i] = w.part[g.index[i]];
+    if (int rc = g.tensor ? launch_tc_linear(xs, w.seg, rows, g.w, g.count, g.ks, parts, st)
+                          : launch_stream_linear(xs, w.seg, rows, g.w, g.count, g.ks, parts, st))
       return rc;
+  }
+  for (int i = 0; i < count; ++i) {
     fa.part[i] = w.part[i];
     fa.out[i] = outs[i];
     fa.ks[i] = w.ks[i];

@@ -41,6 +41,12 @@ struct StreamArgs {
   const uint8_t* st0;
   const uint8_t* st1;
   long long total_rows;  // E * N
+  // NMAT == 3: up to three matrices over the same rows [seg[0], seg[1]), matrix e in
+  // the place of expert e (E of them) with its own row count, output and scales
+  int mtiles[3];
+  int mrows[3];
+  float* mout[3];
+  const uint8_t* mst[3];
 };
 
 // Untiled bulk copy global -> shared (both 16-byte aligned, size % 16 == 0).
@@ -102,7 +108,9 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
                    const __grid_constant__ CUtensorMap tm_s0, const __grid_constant__ CUtensorMap tm_s1,
                    const __grid_constant__ CUtensorMap tm_x8, const __grid_constant__ CUtensorMap tm_x16,
                    const __grid_constant__ CUtensorMap tm_x32, const __grid_constant__ CUtensorMap tm_x64,
+                   const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_s2,
                    const StreamArgs args) {
+  constexpr bool MULTI = NMAT == 3;  // q, k and v projections in one launch; tiles as in the down product
   using C = Cfg<LAYOUT, S, RW, KH_>;
   constexpr int STAGES = C::STAGES;
   constexpr int SET_ROWS = C::SET_ROWS;
@@ -132,13 +140,13 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
     fence_mbar_init();
     int run = 0;
     for (int e = 0; e < args.E; ++e) {
-      const int a = args.seg[e], b = args.seg[e + 1];
+      const int a = args.seg[MULTI ? 0 : e], b = args.seg[MULTI ? 1 : e + 1];
       s_seg[e] = a;
       s_prefix[e] = run;
       const int chunks = (b - a + C::MT - 1) / C::MT;
-      run += chunks * args.ntiles * args.ksplit;
+      run += chunks * (MULTI ? args.mtiles[MULTI ? e : 0] : args.ntiles) * args.ksplit;
     }
-    s_seg[args.E] = args.seg[args.E];
+    s_seg[args.E] = args.seg[MULTI ? 1 : args.E];
     s_prefix[args.E] = run;
   }
   __syncthreads();
@@ -149,14 +157,15 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
     e = 0;
     while (item >= s_prefix[e + 1]) ++e;
     const int local = item - s_prefix[e];
-    const int m = s_seg[e + 1] - s_seg[e];
+    const int seg1 = s_seg[MULTI ? args.E : e + 1];
+    const int m = seg1 - s_seg[e];
     const int chunks = (m + C::MT - 1) / C::MT;
     const int tc = local % chunks;
     const int rest = local / chunks;
     kc = rest % args.ksplit;
     tile = rest / args.ksplit;
     row0 = s_seg[e] + tc * C::MT;
-    rows = min(C::MT, s_seg[e + 1] - row0);
+    rows = min(C::MT, seg1 - row0);
   };
 
   if (warp == C::ACTIVE) {
@@ -183,16 +192,17 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
           const int k0 = (kc * args.stages_per_item + st) * KT;
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            const CUtensorMap* tw = (NMAT == 2 && r == 1) ? &tm_w1 : &tm_w0;
-            const CUtensorMap* ts = (NMAT == 2 && r == 1) ? &tm_s1 : &tm_s0;
-            const int grow = e * args.N + n0 + (NMAT == 2 ? 0 : SET_ROWS * r);
+            const CUtensorMap* tw = (NMAT == 2 && r == 1) || (MULTI && e == 1) ? &tm_w1 : MULTI && e == 2 ? &tm_w2 : &tm_w0;
+            const CUtensorMap* ts = (NMAT == 2 && r == 1) || (MULTI && e == 1) ? &tm_s1 : MULTI && e == 2 ? &tm_s2 : &tm_s0;
+            const int grow = (MULTI ? 0 : e * args.N) + n0 + (NMAT == 2 ? 0 : SET_ROWS * r);
             if constexpr (LAYOUT == B200MOE_LAYOUT_Q8_0) {
               tma_load_2d(sb + r * C::WSET, tw, k0, grow, fb);
               tma_load_2d(sb + r * C::WSET + SET_ROWS * 128, tw, k0 + 128, grow, fb);
-              if (args.st0 != nullptr) {
-                const uint8_t* sp = (NMAT == 2 && r == 1) ? args.st1 : args.st0;
+              const uint8_t* sp = MULTI ? args.mst[MULTI ? e : 0] : (NMAT == 2 && r == 1) ? args.st1 : args.st0;
+              if (sp != nullptr) {
+                const long long total_rows = MULTI ? args.mrows[MULTI ? e : 0] : args.total_rows;
                 bulk_load(sb + C::OFF_S + r * C::SSET,
-                          sp + (static_cast<long long>(k0 / KT) * args.total_rows + grow) * 16,
+                          sp + (static_cast<long long>(k0 / KT) * total_rows + grow) * 16,
                           C::SSET, fb);
               } else {
                 tma_load_2d(sb + C::OFF_S + r * C::SSET, ts, (k0 / 32) * 2, grow, fb);
@@ -431,9 +441,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
           static_cast<__half*>(args.out)[static_cast<size_t>(tok) * args.N + col] =
               to_half_sat(a * up, args.status);
         } else {
-          float* outp = static_cast<float*>(args.out) +
-                        static_cast<size_t>(kc) * args.P * args.N +
-                        static_cast<size_t>(tok) * args.N + tile * (2 * SET_ROWS) + rsub;
+          const size_t N = static_cast<size_t>(MULTI ? args.mrows[MULTI ? e : 0] : args.N);
+          float* outp = (MULTI ? args.mout[MULTI ? e : 0] : static_cast<float*>(args.out)) +
+                        static_cast<size_t>(kc) * args.P * N +
+                        static_cast<size_t>(tok) * N + tile * (2 * SET_ROWS) + rsub;
           outp[0] = acc[0][s][c];
           outp[SET_ROWS] = acc[1][s][c];
         }
@@ -454,7 +465,7 @@ int launch_t(const CUtensorMap* maps, const StreamArgs& a, cudaStream_t st) {
     configured[dev] = true;
   }
   kern<<<sm_count(), C::THREADS, C::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                             maps[6], maps[7], a);
+                                             maps[6], maps[7], maps[8], maps[9], a);
   B200_CHECK_CUDA(cudaGetLastError());
   return B200MOE_OK;
 }
@@ -597,7 +608,7 @@ int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max
       if (S > 2) S = 2;
     }
   }
-  CUtensorMap maps[8];
+  CUtensorMap maps[10] = {};
   if (int rc = weight_maps(gate, &maps[0], &maps[2], set_rows)) return rc;
   if (int rc = weight_maps(up, &maps[1], &maps[3], set_rows)) return rc;
   if (int rc = token_maps(maps, xs, pairs, static_cast<uint64_t>(gate->cols) * 2, S)) return rc;
@@ -645,7 +656,7 @@ int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_
     if (S == 4) S = 2;
     else if (S == 8 && max_segment <= 64) S = 4;
   }
-  CUtensorMap maps[8];
+  CUtensorMap maps[10] = {};
   if (int rc = weight_maps(down, &maps[0], &maps[2])) return rc;
   maps[1] = maps[0];
   maps[3] = maps[2];
@@ -666,6 +677,61 @@ int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_
   if (down->layout == B200MOE_LAYOUT_F16) return launch_s<B200MOE_LAYOUT_F16, 1, 4, 2>(S, maps, a, st);
   return wide ? launch_w<B200MOE_LAYOUT_Q4_K, 1>(S, maps, a, st)
               : launch_s<B200MOE_LAYOUT_Q4_K, 1, 4, 2>(S, maps, a, st);
+}
+
+// ---- several matrices over the same rows (dense quantised linears) -----------
+// k split shared by the matrices: waves of items, each its stages and about two for
+// the boundary.  One B200, 1..16 rows, K 4096, us at a split of 2 / 4 / 8: 4096 output
+// rows (32 tiles) 10.3 / 8.7 / 10.0, 1024 output rows (8 tiles) 10.3 / 8.3 / 6.2.
+int stream_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows) {
+  int row_tiles = 0;
+  for (int i = 0; i < count; ++i) row_tiles += w[i]->rows / 128;
+  const int stages = w[0]->cols / KT;
+  const int sms = sm_count();
+  const int mt = 8 * pick_s(rows);
+  const int tiles = (rows + mt - 1) / mt * row_tiles;
+  int best = 1, best_cost = 0;
+  for (int ks = 1; ks <= 8; ks *= 2) {
+    if (stages % ks != 0) break;
+    const int cost = (tiles * ks + sms - 1) / sms * (stages / ks + 2);
+    if (ks == 1 || cost < best_cost) { best_cost = cost; best = ks; }
+  }
+  return best;
+}
+
+// outs[i] = fp32 [ksplit, rows, w[i]->rows] partial sums of xs w[i]^T; equal layouts and cols.
+int launch_stream_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
+                         int ksplit, float* const* outs, cudaStream_t st) {
+  B200_REQUIRE(count >= 1 && count <= 3, "stream kernel: 1..3 matrices");
+  B200_REQUIRE(ksplit >= 1 && (w[0]->cols / KT) % ksplit == 0, "stream kernel: bad k split %d", ksplit);
+  if (rows == 0) return B200MOE_OK;
+  const int S = pick_s(rows);
+  CUtensorMap maps[10] = {};
+  static constexpr int WMAP[3] = {0, 1, 8}, SMAP[3] = {2, 3, 9};
+  StreamArgs a{};
+  bool tiled_scales = true;
+  for (int i = 0; i < count; ++i) {
+    if (int rc = check_weight(w[i], "linear")) return rc;
+    B200_REQUIRE(w[i]->layout == w[0]->layout && w[i]->cols == w[0]->cols && w[i]->experts == 1 && w[i]->rows % 128 == 0,
+                 "stream kernel: matrices over the same rows need one layout, equal cols and rows %% 128 == 0");
+    if (int rc = weight_maps(w[i], &maps[WMAP[i]], &maps[SMAP[i]])) return rc;
+    a.mrows[i] = w[i]->rows;
+    a.mtiles[i] = w[i]->rows / 128;
+    a.mout[i] = outs[i];
+    a.mst[i] = static_cast<const uint8_t*>(w[i]->sub);
+    tiled_scales = tiled_scales && w[i]->sub != nullptr;
+  }
+  if (w[0]->layout == B200MOE_LAYOUT_Q4_K || !tiled_scales)
+    for (int i = 0; i < count; ++i) a.mst[i] = nullptr;
+  if (int rc = token_maps(maps, xs, rows, static_cast<uint64_t>(w[0]->cols) * 2, S)) return rc;
+  a.seg = seg; a.E = count; a.K = w[0]->cols; a.ksplit = ksplit;
+  a.stages_per_item = w[0]->cols / KT / ksplit;
+  a.P = rows; a.status = device_status_ptr();
+  if (a.status == nullptr) return B200MOE_ERR_CUDA;
+  const bool wide = use_wide(w[0]->layout, S);
+  if (w[0]->layout == B200MOE_LAYOUT_Q8_0)
+    return wide ? launch_w<B200MOE_LAYOUT_Q8_0, 3>(S, maps, a, st) : launch_s<B200MOE_LAYOUT_Q8_0, 3, 4, 2>(S, maps, a, st);
+  return wide ? launch_w<B200MOE_LAYOUT_Q4_K, 3>(S, maps, a, st) : launch_s<B200MOE_LAYOUT_Q4_K, 3, 4, 2>(S, maps, a, st);
 }
 
 void set_stream_wide(int mode) { g_stream_wide = mode; }

@@ -119,6 +119,12 @@ struct TcArgs {
   const uint8_t* st0;
   const uint8_t* st1;
   long long total_rows;
+  // NMAT == 3: up to three matrices over the same rows [seg[0], seg[1]), matrix e in
+  // the place of expert e (E of them) with its own row count, output and scales
+  int mtiles[3];
+  int mrows[3];
+  float* mout[3];
+  const uint8_t* mst[3];
 };
 
 __device__ __forceinline__ void tc_bulk_load(uint32_t dst, const void* src, uint32_t bytes,
@@ -242,7 +248,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
                const __grid_constant__ CUtensorMap tm_x16, const __grid_constant__ CUtensorMap tm_x32,
                const __grid_constant__ CUtensorMap tm_x64, const __grid_constant__ CUtensorMap tm_x96,
                const __grid_constant__ CUtensorMap tm_x128, const __grid_constant__ CUtensorMap tm_x192,
+               const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_s2,
                const TcArgs args) {
+  constexpr bool MULTI = NMAT == 3;  // q, k and v projections in one launch; tiles as in the down product
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_seg[TC_MAX_E + 1];
   __shared__ int s_prefix[TC_MAX_E + 1];
@@ -289,12 +297,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     fence_mbar_init();
     int run = 0;
     for (int e = 0; e < args.E; ++e) {
-      const int a = args.seg[e], b = args.seg[e + 1];
+      const int a = args.seg[MULTI ? 0 : e], b = args.seg[MULTI ? 1 : e + 1];
       s_seg[e] = a;
       s_prefix[e] = run;
-      run += ((b - a + args.tok_tile - 1) / args.tok_tile) * args.ntiles * args.ksplit;
+      run += ((b - a + args.tok_tile - 1) / args.tok_tile) * (MULTI ? args.mtiles[MULTI ? e : 0] : args.ntiles) * args.ksplit;
     }
-    s_seg[args.E] = args.seg[args.E];
+    s_seg[args.E] = args.seg[MULTI ? 1 : args.E];
     s_prefix[args.E] = run;
   }
   if (warp == TC_WARP_MMA) {
@@ -313,19 +321,21 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const uint32_t WSET_BYTES = set_rows * (Q4 ? 64 : 128);  // one set, 128 k
   const uint32_t SSET_BYTES = set_rows * (Q4 ? 32 : 16);   // one set, 256 k
 
-  // tile -> (expert, row tile | k partition << 16, first token row, token rows, MMA N)
+  // tile -> (expert, row tile | k partition << 16 | matrix << 24, first token row, token rows, MMA N)
   auto decode = [&](int tile, int& e, int& nt, int& row0, int& rows, int& ncols) {
     e = 0;
     while (tile >= s_prefix[e + 1]) ++e;
     const int local = tile - s_prefix[e];
-    const int m = s_seg[e + 1] - s_seg[e];
+    const int seg0 = s_seg[e], seg1 = s_seg[MULTI ? args.E : e + 1];
+    const int m = seg1 - seg0;
     const int mtiles = (m + args.tok_tile - 1) / args.tok_tile;
     const int mt = local % mtiles;
     const int rest = local / mtiles;
     nt = (rest / args.ksplit) | ((rest % args.ksplit) << 16);
+    if constexpr (MULTI) nt |= e << 24;
     const int per = ((m + mtiles - 1) / mtiles + 15) & ~15;  // balanced, multiple of 16
-    row0 = s_seg[e] + mt * per;
-    rows = min(per, s_seg[e + 1] - row0);
+    row0 = seg0 + mt * per;
+    rows = min(per, seg1 - row0);
     if (rows < 0) rows = 0;
     ncols = (max(rows, 1) + 15) & ~15;
   };
@@ -338,9 +348,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         int e, nt, row0, rows, ncols;
         decode(tile, e, nt, row0, rows, ncols);
-        const int kbase = (nt >> 16) * stages_per_tile * TC_KT;
+        const int kbase = ((nt >> 16) & 0xff) * stages_per_tile * TC_KT;
         nt &= 0xffff;
-        const int grow0 = e * args.N + nt * (NMAT == 2 ? args.row_tile : 2 * TC_ROWS);
+        const CUtensorMap* const mw0 = MULTI && e == 1 ? &tm_w1 : MULTI && e == 2 ? &tm_w2 : &tm_w0;
+        const CUtensorMap* const ms0 = MULTI && e == 1 ? &tm_s1 : MULTI && e == 2 ? &tm_s2 : &tm_s0;
+        const CUtensorMap* const mw1 = NMAT == 2 ? &tm_w1 : mw0;
+        const CUtensorMap* const ms1 = NMAT == 2 ? &tm_s1 : ms0;
+        const uint8_t* const st0 = MULTI ? args.mst[MULTI ? e : 0] : args.st0;
+        const uint8_t* const st1 = NMAT == 2 ? args.st1 : st0;
+        const long long total_rows = MULTI ? args.mrows[MULTI ? e : 0] : args.total_rows;
+        const int grow0 = (MULTI ? 0 : e * args.N) + nt * (NMAT == 2 ? args.row_tile : 2 * TC_ROWS);
         const int grow1 = NMAT == 2 ? grow0 : grow0 + TC_ROWS;
         for (int st = 0; st < stages_per_tile; st += 2, n += 2) {
           const int k0 = kbase + st * TC_KT;
@@ -353,15 +370,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             const uint32_t sb = sfull + 8u * ss;
             mbar_expect_tx(sb, 2 * SSET_BYTES);
             if constexpr (Q4) {
-              tma_load_2d(sdst, &tm_s0, (k0 / 32) * 4, grow0, sb);
-              tma_load_2d(sdst + TC_SSET, NMAT == 2 ? &tm_s1 : &tm_s0, (k0 / 32) * 4, grow1, sb);
-            } else if (args.st0 != nullptr) {
-              const long long goff = static_cast<long long>(k0 / 256) * args.total_rows;
-              tc_bulk_load(sdst, args.st0 + (goff + grow0) * 16, SSET_BYTES, sb);
-              tc_bulk_load(sdst + TC_SSET, (NMAT == 2 ? args.st1 : args.st0) + (goff + grow1) * 16, SSET_BYTES, sb);
+              tma_load_2d(sdst, ms0, (k0 / 32) * 4, grow0, sb);
+              tma_load_2d(sdst + TC_SSET, ms1, (k0 / 32) * 4, grow1, sb);
+            } else if (st0 != nullptr) {
+              const long long goff = static_cast<long long>(k0 / 256) * total_rows;
+              tc_bulk_load(sdst, st0 + (goff + grow0) * 16, SSET_BYTES, sb);
+              tc_bulk_load(sdst + TC_SSET, st1 + (goff + grow1) * 16, SSET_BYTES, sb);
             } else {
-              tma_load_2d(sdst, &tm_s0, (k0 / 32) * 2, grow0, sb);
-              tma_load_2d(sdst + TC_SSET, NMAT == 2 ? &tm_s1 : &tm_s0, (k0 / 32) * 2, grow1, sb);
+              tma_load_2d(sdst, ms0, (k0 / 32) * 2, grow0, sb);
+              tma_load_2d(sdst + TC_SSET, ms1, (k0 / 32) * 2, grow1, sb);
             }
           }
           const uint32_t wi = n >> 1;
@@ -371,8 +388,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           const uint32_t wdst = smem_base + ws * TC_WSLOT;
           const uint32_t wb = wfull + 8u * ws;
           mbar_expect_tx(wb, 2 * WSET_BYTES);
-          tma_load_2d(wdst, &tm_w0, Q4 ? k0 / 2 : k0, grow0, wb);
-          tma_load_2d(wdst + TC_WSET, NMAT == 2 ? &tm_w1 : &tm_w0, Q4 ? k0 / 2 : k0, grow1, wb);
+          tma_load_2d(wdst, mw0, Q4 ? k0 / 2 : k0, grow0, wb);
+          tma_load_2d(wdst + TC_WSET, mw1, Q4 ? k0 / 2 : k0, grow1, wb);
         }
       }
       // do not leave while copies may still land in this CTA's shared memory
@@ -401,7 +418,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           const int xs = n % TC_XSLOTS;
           if (!mbar_wait(xempty + 8u * xs, ((n / TC_XSLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
           const uint32_t xb = xfull + 8u * xs;
-          const int x0 = ((nt >> 16) * stages_per_tile + st) * TC_KT * 2;
+          const int x0 = (((nt >> 16) & 0xff) * stages_per_tile + st) * TC_KT * 2;
           mbar_expect_tx(xb, 2 * xbytes);
           tma_load_2d(x_base + xs * TC_XSLOT, tx, x0, row0, xb);
           tma_load_2d(x_base + xs * TC_XSLOT + TC_XSUB, tx, x0 + TC_KT * 2, row0, xb);
@@ -524,9 +541,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         }
         if (amax >= 65520.0f) atomicOr(args.status, DEV_WARN_SATURATED);
       } else {
-        float* obase = static_cast<float*>(args.out) + static_cast<size_t>(nt >> 16) * args.P * args.N +
-                       static_cast<size_t>(row0) * args.N + (nt & 0xffff) * (2 * TC_ROWS) + row;
-        const size_t ostride = static_cast<size_t>(args.N);
+        const int mat = MULTI ? nt >> 24 : 0;
+        const size_t ostride = static_cast<size_t>(MULTI ? args.mrows[mat] : args.N);
+        float* obase = (MULTI ? args.mout[mat] : static_cast<float*>(args.out)) +
+                       static_cast<size_t>((nt >> 16) & 0xff) * args.P * ostride +
+                       static_cast<size_t>(row0) * ostride + (nt & 0xffff) * (2 * TC_ROWS) + row;
         for (int c0 = (grp * 2 + set) * 16; c0 < ncols; c0 += 64) {
           uint32_t g[16], u[16];
           tmem_ld16(tmem + lane_addr + TC_COL_ACC0 + c0, g);
@@ -678,7 +697,7 @@ int tc_launch_n(const CUtensorMap* maps, const TcArgs& a, cudaStream_t st) {
     configured[dev] = true;
   }
   kern<<<sm_count(), TC_THREADS, G::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                                maps[6], maps[7], maps[8], maps[9], a);
+                                                maps[6], maps[7], maps[8], maps[9], maps[10], maps[11], a);
   B200_CHECK_CUDA(cudaGetLastError());
   return B200MOE_OK;
 }
@@ -792,7 +811,7 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
   TcArgs a{};
   a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, gate->experts);
   a.row_tile = tc_row_tile(gate->rows, tc_expected_token_tiles(pairs, gate->experts, a.tok_tile), a.tok_tile);
-  CUtensorMap maps[10];
+  CUtensorMap maps[12] = {};
   if (int rc = tc_weight_map(gate, &maps[0], &maps[2], a.row_tile)) return rc;
   if (int rc = tc_weight_map(up, &maps[1], &maps[3], a.row_tile)) return rc;
   if (int rc = tc_token_maps(maps, xs, pairs, static_cast<uint64_t>(gate->cols) * 2)) return rc;
@@ -839,7 +858,7 @@ int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile
   B200_REQUIRE(down->rows % (2 * TC_ROWS) == 0, "tensor kernel: hidden (%d) must be a multiple of 256",
                down->rows);
   if (pairs == 0) return B200MOE_OK;
-  CUtensorMap maps[10];
+  CUtensorMap maps[12] = {};
   if (int rc = tc_weight_map(down, &maps[0], &maps[2])) return rc;
   maps[1] = maps[0];
   maps[3] = maps[2];
@@ -857,6 +876,86 @@ int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile
   if (down->layout == B200MOE_LAYOUT_Q4_K) return tc_launch<B200MOE_LAYOUT_Q4_K, 1>(maps, a, st);
   if (down->sub != nullptr) a.st0 = a.st1 = static_cast<const uint8_t*>(down->sub);
   return tc_launch<B200MOE_LAYOUT_Q8_0, 1>(maps, a, st);
+}
+
+// ---- several matrices over the same rows (dense quantised linears) -----------
+namespace {
+// Token tile for one matrix of `row_tiles` 256-row tiles: the row count is exact, so
+// the last wave can be, too.  Cost of a wave in clocks per 64-k stage: the MMAs of the
+// balanced tile (4 per token), no less than the ~620 that the dequant warps take.
+// 4096 rows x 16 tiles on 148 SMs: 192-row tiles are 352 items = 3 waves of 768,
+// 160-row tiles 416 items = 3 waves of 640.
+int tc_linear_tok_tile(int rows, int row_tiles) {
+  const int narrow = tc_pick_tok_tile(TC_NTOK, rows, 1);
+  if (narrow <= 128) return narrow;
+  const int sms = sm_count();
+  int best = TC_NTOK;
+  double best_cost = 0.0;
+  for (int t = TC_NTOK; t >= 128; t -= 16) {
+    const int mt = (rows + t - 1) / t;
+    const int n = ((rows + mt - 1) / mt + 15) & ~15;
+    const int waves = (mt * row_tiles + sms - 1) / sms;
+    const double cost = waves * ((4 * n > 620 ? 4 * n : 620) + 60);
+    if (t == TC_NTOK || cost < 0.98 * best_cost) { best_cost = cost; best = t; }
+  }
+  return best;
+}
+}  // namespace
+
+// k split shared by the matrices: the cost of tc_down_ksplit with their tiles together.
+int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows) {
+  int row_tiles = 0;
+  long long out_rows = 0;
+  for (int i = 0; i < count; ++i) { row_tiles += w[i]->rows / (2 * TC_ROWS); out_rows += w[i]->rows; }
+  const int stages = w[0]->cols / TC_KT;
+  const int sms = sm_count();
+  const int tok = tc_linear_tok_tile(rows, row_tiles);
+  const double tiles = static_cast<double>((rows + tok - 1) / tok) * row_tiles;
+  const double part = static_cast<double>(rows) * out_rows * 8.0 / 6.5e6 / 0.4;
+  int best = 1;
+  double best_cost = 0.0;
+  for (int ks = 1; ks <= 8; ks *= 2) {
+    if (stages % (4 * ks) != 0) break;
+    const double cost = ceil(tiles * ks / sms) * (stages / ks + 3) + ks * part;
+    if (ks == 1 || cost < 0.98 * best_cost) { best_cost = cost; best = ks; }
+  }
+  return best;
+}
+
+// outs[i] = fp32 [ksplit, rows, w[i]->rows] partial sums of xs w[i]^T; equal layouts and cols.
+int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
+                     int ksplit, float* const* outs, cudaStream_t st) {
+  B200_REQUIRE(count >= 1 && count <= 3, "tensor kernel: 1..3 matrices");
+  if (rows == 0) return B200MOE_OK;
+  CUtensorMap maps[12] = {};
+  static constexpr int WMAP[3] = {0, 1, 10}, SMAP[3] = {2, 3, 11};
+  TcArgs a{};
+  int row_tiles = 0;
+  bool tiled_scales = true;
+  for (int i = 0; i < count; ++i) {
+    if (int rc = tc_check(w[i], "linear")) return rc;
+    B200_REQUIRE(w[i]->experts == 1 && w[i]->layout == w[0]->layout && w[i]->cols == w[0]->cols &&
+                     w[i]->rows % (2 * TC_ROWS) == 0,
+                 "tensor kernel: matrices over the same rows need one layout, equal cols and rows %% 256 == 0");
+    if (int rc = tc_weight_map(w[i], &maps[WMAP[i]], &maps[SMAP[i]])) return rc;
+    a.mrows[i] = w[i]->rows;
+    a.mtiles[i] = w[i]->rows / (2 * TC_ROWS);
+    a.mout[i] = outs[i];
+    a.mst[i] = static_cast<const uint8_t*>(w[i]->sub);
+    row_tiles += a.mtiles[i];
+    tiled_scales = tiled_scales && w[i]->sub != nullptr;
+  }
+  if (w[0]->layout == B200MOE_LAYOUT_Q4_K || !tiled_scales)
+    for (int i = 0; i < count; ++i) a.mst[i] = nullptr;
+  if (int rc = tc_token_maps(maps, xs, rows, static_cast<uint64_t>(w[0]->cols) * 2)) return rc;
+  B200_REQUIRE(ksplit >= 1 && (w[0]->cols / TC_KT) % (4 * ksplit) == 0, "tensor kernel: bad k split %d", ksplit);
+  a.seg = seg; a.E = count; a.K = w[0]->cols; a.P = rows; a.ksplit = ksplit;
+  a.row_tile = TC_ROWS;
+  a.tok_tile = tc_linear_tok_tile(rows, row_tiles);
+  a.status = device_status_ptr();
+  if (a.status == nullptr) return B200MOE_ERR_CUDA;
+  return w[0]->layout == B200MOE_LAYOUT_Q4_K ? tc_launch<B200MOE_LAYOUT_Q4_K, 3>(maps, a, st)
+                                             : tc_launch<B200MOE_LAYOUT_Q8_0, 3>(maps, a, st);
 }
 
 }  // namespace b200moe
