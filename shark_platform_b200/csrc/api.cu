@@ -222,6 +222,45 @@ inline void prof_mark(int call, int idx, cudaStream_t st) {
   if (call >= 0) cudaEventRecord(g_prof.ev[call][idx], st);
 }
 
+int gate_up_impl(const void* xs, const int32_t* seg_offsets, int32_t pairs, int32_t max_segment,
+                 const b200moe_weight_t* gate, const b200moe_weight_t* up, int activation, int regime,
+                 int32_t out_kperm, int prefetch, void* a_out, void* stream) {
+  B200_REQUIRE(gate && up && seg_offsets, "gate_up: NULL argument");
+  B200_REQUIRE(pairs == 0 || (xs && a_out), "gate_up: NULL buffer");
+  B200_REQUIRE(activation == B200MOE_ACT_SILU || activation == B200MOE_ACT_GELU,
+               "gate_up: unknown activation %d", activation);
+  int r = pick_regime(regime, gate, max_segment, false);
+  // shapes the pair kernel cannot tile go to the single-CTA tensor kernel
+  if (r == B200MOE_REGIME_TENSOR_PAIR && !(tc_pair_supported_gate_up(gate) && tc_pair_supported_gate_up(up)))
+    r = B200MOE_REGIME_TENSOR;
+  if (r == B200MOE_REGIME_TENSOR_PAIR)
+    return launch_tc_pair_gate_up(xs, seg_offsets, pairs, 192, gate, up, activation, out_kperm, a_out,
+                                  static_cast<cudaStream_t>(stream));
+  if (r == B200MOE_REGIME_TENSOR) {
+    return launch_tc_gate_up(xs, seg_offsets, pairs, g_token_tile, gate, up, activation, out_kperm, prefetch, a_out,
+                             static_cast<cudaStream_t>(stream));
+  }
+  return launch_stream_gate_up(xs, seg_offsets, pairs, max_segment, gate, up, activation,
+                               out_kperm, prefetch, a_out, static_cast<cudaStream_t>(stream));
+}
+
+int down_impl(const void* a, const int32_t* seg_offsets, int32_t pairs, int32_t max_segment,
+              const b200moe_weight_t* down, int regime, int32_t ksplit, int prefetch, float* d_out, void* stream) {
+  B200_REQUIRE(down && seg_offsets, "down: NULL argument");
+  B200_REQUIRE(pairs == 0 || (a && d_out), "down: NULL buffer");
+  B200_REQUIRE(ksplit >= 1, "down: ksplit must come from b200moe_down_ksplit");
+  int r = pick_regime(regime, down, max_segment, true);
+  if (r == B200MOE_REGIME_TENSOR_PAIR && !tc_pair_supported_down(down)) r = B200MOE_REGIME_TENSOR;
+  if (r == B200MOE_REGIME_TENSOR_PAIR)
+    return launch_tc_pair_down(a, seg_offsets, pairs, 192, down, ksplit, d_out,
+                               static_cast<cudaStream_t>(stream));
+  if (r == B200MOE_REGIME_TENSOR)
+    return launch_tc_down(a, seg_offsets, pairs, g_token_tile, down, ksplit, prefetch, d_out,
+                          static_cast<cudaStream_t>(stream));
+  return launch_stream_down(a, seg_offsets, pairs, max_segment, down, ksplit, prefetch, d_out,
+                            static_cast<cudaStream_t>(stream));
+}
+
 }  // namespace
 }  // namespace b200moe
 
@@ -341,23 +380,8 @@ int b200moe_gate_up(const void* xs, const int32_t* seg_offsets, int32_t pairs,
                     int32_t max_segment, const b200moe_weight_t* gate,
                     const b200moe_weight_t* up, int activation, int regime, int32_t out_kperm,
                     void* a_out, void* stream) {
-  B200_REQUIRE(gate && up && seg_offsets, "gate_up: NULL argument");
-  B200_REQUIRE(pairs == 0 || (xs && a_out), "gate_up: NULL buffer");
-  B200_REQUIRE(activation == B200MOE_ACT_SILU || activation == B200MOE_ACT_GELU,
-               "gate_up: unknown activation %d", activation);
-  int r = pick_regime(regime, gate, max_segment, false);
-  // shapes the pair kernel cannot tile go to the single-CTA tensor kernel
-  if (r == B200MOE_REGIME_TENSOR_PAIR && !(tc_pair_supported_gate_up(gate) && tc_pair_supported_gate_up(up)))
-    r = B200MOE_REGIME_TENSOR;
-  if (r == B200MOE_REGIME_TENSOR_PAIR)
-    return launch_tc_pair_gate_up(xs, seg_offsets, pairs, 192, gate, up, activation, out_kperm, a_out,
-                                  static_cast<cudaStream_t>(stream));
-  if (r == B200MOE_REGIME_TENSOR) {
-    return launch_tc_gate_up(xs, seg_offsets, pairs, g_token_tile, gate, up, activation, out_kperm, a_out,
-                             static_cast<cudaStream_t>(stream));
-  }
-  return launch_stream_gate_up(xs, seg_offsets, pairs, max_segment, gate, up, activation,
-                               out_kperm, a_out, static_cast<cudaStream_t>(stream));
+  return gate_up_impl(xs, seg_offsets, pairs, max_segment, gate, up, activation, regime, out_kperm, PREFETCH_NONE,
+                      a_out, stream);
 }
 
 int b200moe_down_ksplit(const b200moe_weight_t* down, int32_t pairs, int32_t max_segment,
@@ -373,19 +397,7 @@ int b200moe_down_ksplit(const b200moe_weight_t* down, int32_t pairs, int32_t max
 int b200moe_down(const void* a, const int32_t* seg_offsets, int32_t pairs, int32_t max_segment,
                  const b200moe_weight_t* down, int regime, int32_t ksplit, float* d_out,
                  void* stream) {
-  B200_REQUIRE(down && seg_offsets, "down: NULL argument");
-  B200_REQUIRE(pairs == 0 || (a && d_out), "down: NULL buffer");
-  B200_REQUIRE(ksplit >= 1, "down: ksplit must come from b200moe_down_ksplit");
-  int r = pick_regime(regime, down, max_segment, true);
-  if (r == B200MOE_REGIME_TENSOR_PAIR && !tc_pair_supported_down(down)) r = B200MOE_REGIME_TENSOR;
-  if (r == B200MOE_REGIME_TENSOR_PAIR)
-    return launch_tc_pair_down(a, seg_offsets, pairs, 192, down, ksplit, d_out,
-                               static_cast<cudaStream_t>(stream));
-  if (r == B200MOE_REGIME_TENSOR)
-    return launch_tc_down(a, seg_offsets, pairs, g_token_tile, down, ksplit, d_out,
-                          static_cast<cudaStream_t>(stream));
-  return launch_stream_down(a, seg_offsets, pairs, max_segment, down, ksplit, d_out,
-                            static_cast<cudaStream_t>(stream));
+  return down_impl(a, seg_offsets, pairs, max_segment, down, regime, ksplit, PREFETCH_NONE, d_out, stream);
 }
 
 int b200moe_exchange_plan(const int32_t* counts, int32_t world, int32_t experts_local,
@@ -459,12 +471,14 @@ int b200moe_layer_forward(const b200moe_layer_t* L, const void* h, void* y, int 
       return rc;
   }
   prof_mark(pc, 3, st);
-  if (int rc = b200moe_gate_up(w.xs, w.seg, pairs, tokens, &L->gate, &L->up, L->activation, regime,
-                               kp_mid, w.a, stream))
+  // With four pairs per expert or more all experts are most likely active: gate/up
+  // starts fetching before the routing is known.
+  if (int rc = gate_up_impl(w.xs, w.seg, pairs, tokens, &L->gate, &L->up, L->activation, regime, kp_mid,
+                            pairs >= 4 * E ? PREFETCH_ALL_EXPERTS : PREFETCH_NONE, w.a, stream))
     return rc;
   prof_mark(pc, 4, st);
   const int ks = b200moe_down_ksplit(&L->down, pairs, tokens, regime);
-  if (int rc = b200moe_down(w.a, w.seg, pairs, tokens, &L->down, regime, ks, w.dpart, stream)) return rc;
+  if (int rc = down_impl(w.a, w.seg, pairs, tokens, &L->down, regime, ks, PREFETCH_SEGMENTS, w.dpart, stream)) return rc;
   prof_mark(pc, 5, st);
   if (int rc = launch_combine(w.dpart, B200MOE_DT_F32, ks, pairs, w.inv, w.gates, h, io_dtype,
                               tokens, L, 1, y, io_dtype, st))

@@ -45,6 +45,11 @@ int make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, uin
 int make_tmap_2d_sw(CUtensorMap* out, const void* base, uint64_t rows, uint64_t row_bytes,
                     uint32_t box_rows, uint32_t box_bytes, int swizzle_bytes);
 
+// What a GEMM kernel of a layer call may prefetch into L2 while the kernel before it
+// still runs: nothing, the weights its first work item has if every expert turns out
+// to be active (the routing is not known yet), or those of the segments (known).
+enum : int { PREFETCH_NONE = 0, PREFETCH_ALL_EXPERTS = 1, PREFETCH_SEGMENTS = 2 };
+
 // Error bits written to the device status word.
 enum : int32_t {
   DEV_ERR_WAIT_TIMEOUT = 1,  // a bounded mbarrier wait gave up
@@ -56,6 +61,32 @@ enum : int32_t {
 
 // -------------------------------------------------------------- device side
 #ifdef __CUDACC__
+
+// Launch of a kernel that may start while the one before it in the stream still runs
+// (programmatic dependent launch).  The kernel calls grid_dep_wait() in every thread
+// before it touches anything an earlier kernel writes or reads: until then it sets up
+// barriers and tensor memory and at most prefetches weights into L2, so the start-up
+// of each kernel of a layer hides behind the tail of the one before.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// Waits until the kernels before this one in the stream have completed and their
+// writes are visible.  A no-op in a kernel launched the ordinary way.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start once every block has said so (or ended).
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -152,6 +183,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tma
       "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(bar)
       : "memory");
+}
+
+// The same box into L2 only.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int32_t x, int32_t y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(
+                   reinterpret_cast<uint64_t>(tmap)),
+               "r"(x), "r"(y)
+               : "memory");
 }
 
 __device__ __forceinline__ void lds128(uint32_t addr, uint32_t (&v)[4]) {

@@ -38,9 +38,9 @@ int launch_gguf_q4k(const uint8_t* raw, long long blocks, void* d, void* dmin, u
 int stream_down_ksplit(const b200moe_weight_t* down, int pairs);
 int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max_segment,
                           const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
-                          int out_kperm, void* a_out, cudaStream_t st);
+                          int out_kperm, int prefetch, void* a_out, cudaStream_t st);
 int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_segment,
-                       const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st);
+                       const b200moe_weight_t* down, int ksplit, int prefetch, float* d_out, cudaStream_t st);
 int stream_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows);
 int launch_stream_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
                          int ksplit, float* const* outs, cudaStream_t st);
@@ -51,10 +51,10 @@ void set_stream_wide(int mode);
 bool tc_supported(const b200moe_weight_t* w, bool down);
 int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_tile,
                       const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
-                      int out_kperm, void* a_out, cudaStream_t st);
+                      int out_kperm, int prefetch, void* a_out, cudaStream_t st);
 int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs);
 int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile,
-                   const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st);
+                   const b200moe_weight_t* down, int ksplit, int prefetch, float* d_out, cudaStream_t st);
 
 int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows);
 int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,

@@ -69,6 +69,8 @@ __global__ void __launch_bounds__(LR_THREADS) linear_rows_kernel(const LinRowsAr
   const int tid = threadIdx.x;
   const size_t base = static_cast<size_t>(blockIdx.x) * a.K;
   const int nvec = a.K / 8;
+  grid_dep_wait();
+  grid_dep_launch();
   if (blockIdx.x == 0 && tid < 2) a.seg[tid] = tid * a.rows;
   if (a.norm_w == nullptr) {
     for (int j = tid; j < nvec; j += LR_THREADS) {
@@ -144,6 +146,8 @@ __device__ __forceinline__ float lin_round(float v, int dt) {
 template <int DT>
 __global__ void __launch_bounds__(256) linear_finish_kernel(const LinFinishArgs a) {
   const long long total = a.vec_end[a.count - 1];
+  grid_dep_wait();
+  grid_dep_launch();
   for (long long vi = blockIdx.x * 256ll + threadIdx.x; vi < total; vi += gridDim.x * 256ll) {
     int o = 0;
     while (vi >= a.vec_end[o]) ++o;
@@ -307,10 +311,12 @@ int b200moe_linear(const void* x, int x_dtype, int32_t rows, const float* norm_w
   LinRowsArgs ra{x, norm_weight, eps, weights[0]->cols, rows, w.plain, w.perm, w.seg};
   // (with nothing to convert one CTA still writes the segment)
   const unsigned row_ctas = (w.plain != nullptr || w.perm != nullptr) ? static_cast<unsigned>(rows) : 1u;
-  if (x_dtype == B200MOE_DT_F32) linear_rows_kernel<B200MOE_DT_F32><<<row_ctas, LR_THREADS, 0, st>>>(ra);
-  else if (x_dtype == B200MOE_DT_F16) linear_rows_kernel<B200MOE_DT_F16><<<row_ctas, LR_THREADS, 0, st>>>(ra);
-  else linear_rows_kernel<B200MOE_DT_BF16><<<row_ctas, LR_THREADS, 0, st>>>(ra);
-  B200_CHECK_CUDA(cudaGetLastError());
+  if (x_dtype == B200MOE_DT_F32)
+    B200_CHECK_CUDA(launch_dependent(linear_rows_kernel<B200MOE_DT_F32>, dim3(row_ctas), dim3(LR_THREADS), 0, st, ra));
+  else if (x_dtype == B200MOE_DT_F16)
+    B200_CHECK_CUDA(launch_dependent(linear_rows_kernel<B200MOE_DT_F16>, dim3(row_ctas), dim3(LR_THREADS), 0, st, ra));
+  else
+    B200_CHECK_CUDA(launch_dependent(linear_rows_kernel<B200MOE_DT_BF16>, dim3(row_ctas), dim3(LR_THREADS), 0, st, ra));
   LinFinishArgs fa{};
   long long run = 0;
   for (int layout : LIN_LAYOUTS) {
@@ -337,10 +343,12 @@ int b200moe_linear(const void* x, int x_dtype, int32_t rows, const float* norm_w
   fa.count = count;
   const long long want = (run + 255) / 256, most = 16ll * sm_count();
   const unsigned ctas = static_cast<unsigned>(want < most ? want : most);
-  if (out_dtype == B200MOE_DT_F32) linear_finish_kernel<B200MOE_DT_F32><<<ctas, 256, 0, st>>>(fa);
-  else if (out_dtype == B200MOE_DT_F16) linear_finish_kernel<B200MOE_DT_F16><<<ctas, 256, 0, st>>>(fa);
-  else linear_finish_kernel<B200MOE_DT_BF16><<<ctas, 256, 0, st>>>(fa);
-  B200_CHECK_CUDA(cudaGetLastError());
+  if (out_dtype == B200MOE_DT_F32)
+    B200_CHECK_CUDA(launch_dependent(linear_finish_kernel<B200MOE_DT_F32>, dim3(ctas), dim3(256), 0, st, fa));
+  else if (out_dtype == B200MOE_DT_F16)
+    B200_CHECK_CUDA(launch_dependent(linear_finish_kernel<B200MOE_DT_F16>, dim3(ctas), dim3(256), 0, st, fa));
+  else
+    B200_CHECK_CUDA(launch_dependent(linear_finish_kernel<B200MOE_DT_BF16>, dim3(ctas), dim3(256), 0, st, fa));
   return B200MOE_OK;
 }
 

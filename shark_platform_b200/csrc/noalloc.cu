@@ -78,7 +78,7 @@ extern "C" int b200moe_down_noalloc(const void* a, const int32_t* seg_offsets, i
   float* scratch = scratch_ptr();
   if (scratch == nullptr) return B200MOE_ERR_CUDA;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (int rc = launch_stream_down(a, seg_offsets, pairs, max_segment, down, ks, scratch, st))
+  if (int rc = launch_stream_down(a, seg_offsets, pairs, max_segment, down, ks, PREFETCH_NONE, scratch, st))
     return rc;
   const long long n = static_cast<long long>(pairs) * down->rows;
   const int blocks = static_cast<int>(n / 256 + 1 < 1184 ? n / 256 + 1 : 1184);

@@ -422,13 +422,17 @@ router_smem_bf16_kernel(const __nv_bfloat16* __restrict__ h, int tokens, int d, 
 // One CTA per token: used for small token counts (decode), where a warp per
 // token leaves most of the GPU idle.  The row stays in registers between the
 // two passes (hidden <= 8192).
-constexpr int RB_THREADS = 256;
-constexpr int RB_MAXV = 4;  // 8-element vectors per thread
+constexpr int RB_THREADS = 512;
+constexpr int RB_MAXV = 2;  // 8-element vectors per thread
 
 // Router for the token of this CTA.  Leaves the normalised row in `x` (this
 // thread's 8-element vectors tid + v*RB_THREADS); writes it as fp16 to xn_row
 // unless that is null; warp 0 writes the token's experts and gates.
-template <typename T>
+// One token is all latency, so there is one round of memory and one reduction: the
+// row, the norm weights and the first eight experts' router weights are fetched
+// together, and the logits are rstd * sum(x * norm_w * router_w), so that they need
+// not wait for the norm's own sum.  `loaded` runs once that round is back.
+template <typename T, typename F>
 __device__ __forceinline__ void router_block_body(const T* __restrict__ row, int d, int E, int k,
                                                   float eps, const float* __restrict__ norm_w,
                                                   const float* __restrict__ rw,
@@ -436,32 +440,60 @@ __device__ __forceinline__ void router_block_body(const T* __restrict__ row, int
                                                   __half* __restrict__ xn_row,
                                                   int32_t* __restrict__ experts_row,
                                                   float* __restrict__ gates_row,
-                                                  float (&x)[RB_MAXV][8]) {
-  __shared__ float s_part[RB_THREADS / 32][8];
+                                                  float (&x)[RB_MAXV][8], F&& loaded) {
+  constexpr int WARPS = RB_THREADS / 32;
+  __shared__ float s_part[WARPS][9];  // eight logit sums, sum of squares
   __shared__ float s_logit[MAX_EXPERTS];
-  __shared__ float s_ss[RB_THREADS / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nvec = d / 8;
-  float ss = 0.f;
-  float nw[RB_MAXV][8];  // norm weights: fetched with the row, not after the reduction (one memory latency less)
+  float nw[RB_MAXV][8];
+  float rstd = 0.f;
+  for (int e0 = 0; e0 < E; e0 += 8) {
+    float acc[9];
 #pragma unroll
-  for (int v = 0; v < RB_MAXV; ++v) {
-    const int j = tid + v * RB_THREADS;
-    if (j < nvec) {
-      load8<T>(row + j * 8, x[v]);
-      load8<float>(norm_w + j * 8, nw[v]);
+    for (int e = 0; e < 9; ++e) acc[e] = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss = fmaf(x[v][i], x[v][i], ss);
+    for (int v = 0; v < RB_MAXV; ++v) {
+      const int j = tid + v * RB_THREADS;
+      if (j < nvec) {
+        if (e0 == 0) {
+          load8<T>(row + j * 8, x[v]);
+          load8<float>(norm_w + j * 8, nw[v]);
+        }
+        float r[8][8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (e0 + e < E) load8<float>(rw + static_cast<size_t>(e0 + e) * d + j * 8, r[e]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          acc[8] = fmaf(x[v][i], x[v][i], acc[8]);
+          const float xw = x[v][i] * nw[v][i];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (e0 + e < E) acc[e] = fmaf(xw, r[e][i], acc[e]);
+        }
+      }
     }
+#pragma unroll
+    for (int e = 0; e < 9; ++e) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+      if (lane == 0) s_part[warp][e] = acc[e];
+    }
+    if (e0 == 0) loaded();
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) tot += s_part[w][8];
+    rstd = 1.0f / sqrtf(tot / static_cast<float>(d) + eps);
+    if (tid < 8 && e0 + tid < E) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) v += s_part[w][tid];
+      s_logit[e0 + tid] = v * rstd + (rb ? rb[e0 + tid] : 0.f);
+    }
+    if (e0 + 8 < E) __syncthreads();  // s_part is rewritten
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if (lane == 0) s_ss[warp] = ss;
-  __syncthreads();
-  float tot = 0.f;
-#pragma unroll
-  for (int w = 0; w < RB_THREADS / 32; ++w) tot += s_ss[w];
-  const float rstd = 1.0f / sqrtf(tot / static_cast<float>(d) + eps);
 #pragma unroll
   for (int v = 0; v < RB_MAXV; ++v) {
     const int j = tid + v * RB_THREADS;
@@ -477,41 +509,11 @@ __device__ __forceinline__ void router_block_body(const T* __restrict__ row, int
       }
     }
   }
-  for (int e0 = 0; e0 < E; e0 += 8) {
-    float acc[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-#pragma unroll
-    for (int v = 0; v < RB_MAXV; ++v) {
-      const int j = tid + v * RB_THREADS;
-      if (j < nvec) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (e0 + e < E) {
-            float r[8];
-            load8<float>(rw + static_cast<size_t>(e0 + e) * d + j * 8, r);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[e] = fmaf(x[v][i], r[i], acc[e]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-      if (lane == 0) s_part[warp][e] = acc[e];
-    }
-    __syncthreads();
-    if (tid < 8 && e0 + tid < E) {
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < RB_THREADS / 32; ++w) v += s_part[w][tid];
-      s_logit[e0 + tid] = v + (rb ? rb[e0 + tid] : 0.f);
-    }
-    __syncthreads();
+  // the logits were written by threads of warp 0, which also selects
+  if (warp == 0) {
+    __syncwarp();
+    router_select(s_logit, lane, E, k, experts_row, gates_row);
   }
-  if (warp == 0) router_select(s_logit, lane, E, k, experts_row, gates_row);
 }
 
 template <typename T>
@@ -523,7 +525,7 @@ router_block_kernel(const T* __restrict__ h, int d, int E, int k, float eps,
   const size_t t = blockIdx.x;
   float x[RB_MAXV][8];
   router_block_body<T>(h + t * d, d, E, k, eps, norm_w, rw, rb, xn_out + t * d,
-                       experts_out + t * k, gates_out + t * k, x);
+                       experts_out + t * k, gates_out + t * k, x, [] {});
 }
 
 // ------------------------------------------------- fused decode front end
@@ -590,7 +592,10 @@ front_fused_kernel(const T* __restrict__ h, int d, int E, int k, float eps,
   const int t = blockIdx.x, tokens = gridDim.x, pairs = tokens * k;
   float x[RB_MAXV][8];
   router_block_body<T>(h + static_cast<size_t>(t) * d, d, E, k, eps, norm_w, rw, rb, nullptr,
-                       experts_out + static_cast<size_t>(t) * k, gates_out + static_cast<size_t>(t) * k, x);
+                       experts_out + static_cast<size_t>(t) * k, gates_out + static_cast<size_t>(t) * k, x,
+                       // gate/up may start once this kernel's own loads are back: its prefetches
+                       // then run beside the selection and the barrier, not against the loads
+                       [] { grid_dep_launch(); });
   if (tid < MAX_EXPERTS) s_total[tid] = 0;
   if (tid < MAX_TOPK) s_rank[tid] = 0;
   if (!front_grid_meet(sync, static_cast<unsigned>(tokens), status)) return;
@@ -1072,6 +1077,7 @@ combine_kernel(const TD* __restrict__ dpart, int ksplit, size_t part_stride,
   const size_t t = blockIdx.x;
   int pos[MAX_TOPK];
   float gate[MAX_TOPK];
+  grid_dep_wait();
 #pragma unroll
   for (int s = 0; s < MAX_TOPK; ++s) {
     pos[s] = s < k ? inv[t * k + s] : -1;
@@ -1147,12 +1153,10 @@ int launch_combine(const void* dpart, int d_dtype, int ksplit, int pairs, const 
   if (!need_row && tokens < 1024) slices = max(1, min(d / COMBINE_THREADS, 2048 / tokens));
   dim3 grid(tokens, slices), block(COMBINE_THREADS);
 #define LAUNCH(TD, TH, TY)                                                                     \
-  combine_kernel<TD, TH, TY><<<grid, block, smem, st>>>(static_cast<const TD*>(dpart), ksplit,   \
-                                                        stride, inv, gates,                      \
-                                                        static_cast<const TH*>(h), d, k,         \
-                                                        L->layer_output_norm_weight,             \
-                                                        L->rms_epsilon, add_residual,            \
-                                                        static_cast<TY*>(y))
+  B200_CHECK_CUDA(launch_dependent(combine_kernel<TD, TH, TY>, grid, block, smem, st,             \
+                                   static_cast<const TD*>(dpart), ksplit, stride, inv, gates,     \
+                                   static_cast<const TH*>(h), d, k, L->layer_output_norm_weight,  \
+                                   L->rms_epsilon, add_residual, static_cast<TY*>(y)))
   const bool dbf = d_dtype == B200MOE_DT_BF16;
   B200_REQUIRE(dbf || d_dtype == B200MOE_DT_F32, "combine: partial rows must be fp32 or bf16");
   if (h_dtype == B200MOE_DT_F32 && y_dtype == B200MOE_DT_F32) {

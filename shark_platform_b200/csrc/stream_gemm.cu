@@ -34,6 +34,7 @@ struct StreamArgs {
   int P;                // rows of the activation / output arrays
   int act;
   int out_kperm;        // gate/up only: permute output columns for a Q4_K down matrix
+  int prefetch;         // PREFETCH_*
   void* out;
   int32_t* status;
   // Q8_0 only: scales transposed to [K/256][rows][8] (16 bytes per row and
@@ -102,6 +103,44 @@ __device__ __forceinline__ __half2 bcast_half(uint32_t v, int sel) {
   return u32_as_h2(__byte_perm(v, v, sel ? 0x3232 : 0x1010));
 }
 
+// L2 prefetch of the first weight stages of this CTA's first work item, before the
+// results of the earlier kernels may be read (see tc_prefetch: stale offsets would only
+// steer it to other rows of the same matrix).
+constexpr int ST_PREFETCH_STAGES = 6;
+template <int LAYOUT, int NMAT, int SET_ROWS, int MT>
+__device__ __forceinline__ void stream_prefetch(const CUtensorMap& tm_w0, const CUtensorMap& tm_w1, const StreamArgs& args) {
+  int item = blockIdx.x, e = 0;
+  if (args.prefetch == PREFETCH_ALL_EXPERTS) {
+    e = item / (args.ntiles * args.ksplit);
+    if (e >= args.E) return;
+    item -= e * args.ntiles * args.ksplit;
+  } else {
+    int a = __ldcg(args.seg);
+    for (;; ++e) {
+      if (e >= args.E) return;
+      const int b = __ldcg(args.seg + e + 1);
+      const int chunks = b > a ? (b - a + MT - 1) / MT : 0;
+      const int items = chunks * args.ntiles * args.ksplit;
+      if (item < items) { item /= chunks; break; }
+      item -= items;
+      a = b;
+    }
+  }
+  const int kc = item % args.ksplit, tile = item / args.ksplit;
+  if (tile < 0 || tile >= args.ntiles) return;
+  const int grow = e * args.N + tile * (NMAT == 2 ? SET_ROWS : 2 * SET_ROWS);
+  // boxes are 128 bytes wide: 128 k of Q8_0, 256 k of Q4_K, 64 k of fp16
+  constexpr int BOXES = LAYOUT == B200MOE_LAYOUT_Q8_0 ? 2 : LAYOUT == B200MOE_LAYOUT_Q4_K ? 1 : 4;
+  for (int st = 0; st < ST_PREFETCH_STAGES && st < args.stages_per_item; ++st)
+#pragma unroll
+    for (int c = 0; c < BOXES; ++c) {
+      const int x = ((kc * args.stages_per_item + st) * BOXES + c) * 128;
+      tma_prefetch_2d(&tm_w0, x, grow);
+      if constexpr (NMAT == 2) tma_prefetch_2d(&tm_w1, x, grow);
+      else tma_prefetch_2d(&tm_w0, x, grow + SET_ROWS);
+    }
+}
+
 template <int LAYOUT, int NMAT, int S, int RW, int KH_>
 __global__ void __launch_bounds__((RW * KH_ + 1) * 32, 1)
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
@@ -138,6 +177,13 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
       mbar_init(empty_bar(s), C::ACTIVE);
     }
     fence_mbar_init();
+  }
+  if (NMAT != 3 && args.prefetch != PREFETCH_NONE && warp == C::ACTIVE && lane == 0)
+    stream_prefetch<LAYOUT, NMAT, SET_ROWS, C::MT>(tm_w0, tm_w1, args);
+  // from here on the results of earlier kernels are read
+  grid_dep_wait();
+  grid_dep_launch();
+  if (tid == 0) {
     int run = 0;
     for (int e = 0; e < args.E; ++e) {
       const int a = args.seg[MULTI ? 0 : e], b = args.seg[MULTI ? 1 : e + 1];
@@ -464,9 +510,7 @@ int launch_t(const CUtensorMap* maps, const StreamArgs& a, cudaStream_t st) {
     B200_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     configured[dev] = true;
   }
-  kern<<<sm_count(), C::THREADS, C::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                             maps[6], maps[7], maps[8], maps[9], a);
-  B200_CHECK_CUDA(cudaGetLastError());
+  B200_CHECK_CUDA(launch_dependent(kern, dim3(sm_count()), dim3(C::THREADS), C::SMEM, st, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], maps[8], maps[9], a));
   return B200MOE_OK;
 }
 
@@ -574,7 +618,7 @@ int stream_down_ksplit(const b200moe_weight_t* down, int pairs) {
 
 int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max_segment,
                           const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
-                          int out_kperm, void* a_out, cudaStream_t st) {
+                          int out_kperm, int prefetch, void* a_out, cudaStream_t st) {
   if (int rc = check_weight(gate, "gate")) return rc;
   if (int rc = check_weight(up, "up")) return rc;
   B200_REQUIRE(gate->layout == up->layout && gate->rows == up->rows && gate->cols == up->cols &&
@@ -615,7 +659,7 @@ int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max
   StreamArgs a{};
   a.seg = seg; a.E = gate->experts; a.N = gate->rows; a.K = gate->cols;
   a.ntiles = gate->rows / set_rows; a.ksplit = 1; a.stages_per_item = gate->cols / KT;
-  a.P = pairs; a.act = act; a.out_kperm = out_kperm; a.out = a_out; a.status = device_status_ptr();
+  a.P = pairs; a.act = act; a.out_kperm = out_kperm; a.prefetch = prefetch; a.out = a_out; a.status = device_status_ptr();
   if (gate->layout == B200MOE_LAYOUT_Q8_0 && gate->sub != nullptr && up->sub != nullptr) {
     a.st0 = static_cast<const uint8_t*>(gate->sub);
     a.st1 = static_cast<const uint8_t*>(up->sub);
@@ -639,7 +683,7 @@ int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max
 }
 
 int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_segment,
-                       const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st) {
+                       const b200moe_weight_t* down, int ksplit, int prefetch, float* d_out, cudaStream_t st) {
   if (int rc = check_weight(down, "down")) return rc;
   B200_REQUIRE(down->rows % 128 == 0,
                "stream kernel: hidden (%d) must be a multiple of 128", down->rows);
@@ -665,7 +709,7 @@ int launch_stream_down(const void* a_in, const int32_t* seg, int pairs, int max_
   a.seg = seg; a.E = down->experts; a.N = down->rows; a.K = down->cols;
   a.ntiles = down->rows / 128; a.ksplit = ksplit;
   a.stages_per_item = down->cols / KT / ksplit;
-  a.P = pairs; a.act = 0; a.out_kperm = 0; a.out = d_out; a.status = device_status_ptr();
+  a.P = pairs; a.act = 0; a.out_kperm = 0; a.prefetch = prefetch; a.out = d_out; a.status = device_status_ptr();
   if (down->layout == B200MOE_LAYOUT_Q8_0 && down->sub != nullptr)
     a.st0 = a.st1 = static_cast<const uint8_t*>(down->sub);
   a.total_rows = static_cast<long long>(down->experts) * down->rows;

@@ -112,6 +112,7 @@ struct TcArgs {
   int P;
   int act;
   int out_kperm;   // gate/up only: interleave output columns for a Q4_K down matrix
+  int prefetch;    // PREFETCH_*
   void* out;
   int32_t* status;
   // scales transposed to [K/256][rows][8] (one contiguous run per row tile and
@@ -241,6 +242,46 @@ __device__ __forceinline__ uint32_t make_idesc(int m, int n) {
   return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// L2 prefetch of the first weight stages of this CTA's first tile, before the results
+// of the earlier kernels may be read.  With PREFETCH_SEGMENTS the segment offsets are
+// those of a kernel that had completed before the one just ahead of us started; they
+// are read past L1 and, should they be stale all the same, only steer the prefetch to
+// other rows of the same matrix.  TC_PREFETCH stages: the ring's and a few more, about
+// what HBM delivers while the previous kernel drains.
+constexpr int TC_PREFETCH_K = 1536;
+template <int LAYOUT, int NMAT>
+__device__ __forceinline__ void tc_prefetch(const CUtensorMap& tm_w0, const CUtensorMap& tm_w1, const TcArgs& args) {
+  constexpr bool Q4 = LAYOUT == B200MOE_LAYOUT_Q4_K;
+  int tile = blockIdx.x, e = 0, kc = 0;
+  if (args.prefetch == PREFETCH_ALL_EXPERTS) {
+    e = tile / (args.ntiles * args.ksplit);
+    if (e >= args.E) return;
+    tile -= e * args.ntiles * args.ksplit;
+  } else {
+    int a = __ldcg(args.seg);
+    for (;; ++e) {
+      if (e >= args.E) return;
+      const int b = __ldcg(args.seg + e + 1);
+      const int mt = b > a ? (b - a + args.tok_tile - 1) / args.tok_tile : 0;
+      const int items = mt * args.ntiles * args.ksplit;
+      if (tile < items) { tile /= mt; break; }
+      tile -= items;
+      a = b;
+    }
+  }
+  kc = tile % args.ksplit;
+  const int nt = tile / args.ksplit;
+  if (nt < 0 || nt >= args.ntiles) return;
+  const int k_part = args.K / args.ksplit;
+  const int grow0 = e * args.N + nt * (NMAT == 2 ? args.row_tile : 2 * TC_ROWS);
+  for (int k = 0; k < TC_PREFETCH_K && k < k_part; k += 128) {
+    const int x = (kc * k_part + k) / (Q4 ? 2 : 1);
+    tma_prefetch_2d(&tm_w0, x, grow0);
+    if constexpr (NMAT == 2) tma_prefetch_2d(&tm_w1, x, grow0);
+    else tma_prefetch_2d(&tm_w0, x, grow0 + TC_ROWS);
+  }
+}
+
 template <int LAYOUT, int NMAT, int NMAX>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
@@ -295,6 +336,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     mbar_init(acc_full_bar, 2);  // both issuers commit
     mbar_init(acc_empty_bar, TC_DQ_WARPS);  // one arrival per dequant warp
     fence_mbar_init();
+  }
+  if (warp == TC_WARP_MMA) {
+    tmem_alloc(smem_u32(&s_tmem), 512);
+    tmem_relinquish();
+  }
+  if (NMAT != 3 && args.prefetch != PREFETCH_NONE && warp == TC_WARP_WPROD && lane == 0) tc_prefetch<LAYOUT, NMAT>(tm_w0, tm_w1, args);
+  // from here on the results of earlier kernels are read
+  grid_dep_wait();
+  grid_dep_launch();
+  if (tid == 0) {
     int run = 0;
     for (int e = 0; e < args.E; ++e) {
       const int a = args.seg[MULTI ? 0 : e], b = args.seg[MULTI ? 1 : e + 1];
@@ -304,10 +355,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     }
     s_seg[args.E] = args.seg[MULTI ? 1 : args.E];
     s_prefix[args.E] = run;
-  }
-  if (warp == TC_WARP_MMA) {
-    tmem_alloc(smem_u32(&s_tmem), 512);
-    tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
@@ -696,9 +743,7 @@ int tc_launch_n(const CUtensorMap* maps, const TcArgs& a, cudaStream_t st) {
     B200_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
     configured[dev] = true;
   }
-  kern<<<sm_count(), TC_THREADS, G::SMEM, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                                maps[6], maps[7], maps[8], maps[9], maps[10], maps[11], a);
-  B200_CHECK_CUDA(cudaGetLastError());
+  B200_CHECK_CUDA(launch_dependent(kern, dim3(sm_count()), dim3(TC_THREADS), G::SMEM, st, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], maps[8], maps[9], maps[10], maps[11], a));
   return B200MOE_OK;
 }
 
@@ -800,7 +845,7 @@ bool tc_supported(const b200moe_weight_t* w, bool down) {
 
 int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_tile,
                       const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
-                      int out_kperm, void* a_out, cudaStream_t st) {
+                      int out_kperm, int prefetch, void* a_out, cudaStream_t st) {
   if (int rc = tc_check(gate, "gate")) return rc;
   if (int rc = tc_check(up, "up")) return rc;
   B200_REQUIRE(gate->rows == up->rows && gate->cols == up->cols && gate->experts == up->experts &&
@@ -819,6 +864,7 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
   a.ntiles = gate->rows / a.row_tile; a.P = pairs; a.act = act;
   a.ksplit = 1;
   a.out_kperm = out_kperm;
+  a.prefetch = a.tok_tile <= 128 ? prefetch : PREFETCH_NONE;
   a.out = a_out; a.status = device_status_ptr();
   a.total_rows = static_cast<long long>(gate->experts) * gate->rows;
   if (a.status == nullptr) return B200MOE_ERR_CUDA;
@@ -853,7 +899,7 @@ int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs) {
 }
 
 int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile,
-                   const b200moe_weight_t* down, int ksplit, float* d_out, cudaStream_t st) {
+                   const b200moe_weight_t* down, int ksplit, int prefetch, float* d_out, cudaStream_t st) {
   if (int rc = tc_check(down, "down")) return rc;
   B200_REQUIRE(down->rows % (2 * TC_ROWS) == 0, "tensor kernel: hidden (%d) must be a multiple of 256",
                down->rows);
@@ -870,6 +916,7 @@ int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile
   a.row_tile = TC_ROWS;
   a.ntiles = down->rows / (2 * TC_ROWS); a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, down->experts); a.P = pairs; a.act = 0;
   a.ksplit = ksplit;
+  a.prefetch = a.tok_tile <= 128 ? prefetch : PREFETCH_NONE;
   a.out = d_out; a.status = device_status_ptr();
   a.total_rows = static_cast<long long>(down->experts) * down->rows;
   if (a.status == nullptr) return B200MOE_ERR_CUDA;
