@@ -461,6 +461,13 @@ int b200moe_layer_forward(const b200moe_layer_t* L, const void* h, void* y, int 
       return rc;
     prof_mark(pc, 1, st);
     prof_mark(pc, 2, st);
+  } else if (front_prefill_supported(tokens, L)) {
+    // two launches, booked under the router stage
+    if (int rc = launch_front_prefill(h, io_dtype, tokens, L, w.experts, w.gates, w.counts, w.seg, w.perm, w.inv,
+                                      kp_in, w.xs, w.xn, st))
+      return rc;
+    prof_mark(pc, 1, st);
+    prof_mark(pc, 2, st);
   } else {
     if (int rc = launch_router(h, io_dtype, tokens, L, w.xn, w.experts, w.gates, st)) return rc;
     prof_mark(pc, 1, st);

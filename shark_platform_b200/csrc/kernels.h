@@ -16,6 +16,11 @@ int launch_front_fused(const void* h, int h_dtype, int tokens, const b200moe_lay
                        int32_t* experts, float* gates, int32_t* counts, int32_t* seg,
                        int32_t* perm, int32_t* inv, int kperm, void* xs, int32_t* status,
                        cudaStream_t st);
+// the same for larger token counts in two launches; scratch: tokens * hidden * 2 bytes
+bool front_prefill_supported(int tokens, const b200moe_layer_t* L);
+int launch_front_prefill(const void* h, int h_dtype, int tokens, const b200moe_layer_t* L, int32_t* experts,
+                         float* gates, int32_t* counts, int32_t* seg, int32_t* perm, int32_t* inv, int kperm,
+                         void* xs, void* scratch, cudaStream_t st);
 int clear_front_sync(cudaStream_t st);
 int launch_exchange_plan(const int32_t* counts, int world, int el, int32_t* seg, int32_t* perm,
                          int32_t* inv, cudaStream_t st);

@@ -9,10 +9,10 @@
 namespace b200moe {
 
 // ------------------------------------------------------------------ router
-// One warp per token.  RMS norm in fp32 (x * 1/sqrt(mean(x^2)+eps), then the
-// norm weight), router logits from the fp32 normalised row, fp32 softmax,
-// top-k by descending probability (ties: lowest expert id) and renormalised
-// gates.  The normalised row is written as fp16 for the expert products.
+// RMS norm in fp32, router logits from the fp32 normalised row, fp32 softmax, top-k by
+// descending probability (ties: lowest expert id) and renormalised gates.  All router
+// kernels compute a logit as rstd * sum((x * norm_w) * router_w) + bias, eight
+// consecutive columns per lane, 256 per warp, warps added in order.
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&v)[8]);
 
@@ -34,120 +34,11 @@ __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, flo
   }
 }
 
-constexpr int ROUTER_WARPS = 8;
 constexpr int MAX_EXPERTS = 64;
 constexpr int MAX_TOPK = 8;
 
-template <typename T>
-__global__ void __launch_bounds__(ROUTER_WARPS * 32)
-router_kernel(const T* __restrict__ h, int tokens, int d, int E, int k, float eps,
-              const float* __restrict__ norm_w, const float* __restrict__ rw,
-              const float* __restrict__ rb, __half* __restrict__ xn_out,
-              int32_t* __restrict__ experts_out, float* __restrict__ gates_out) {
-  __shared__ float s_logit[ROUTER_WARPS][MAX_EXPERTS];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * ROUTER_WARPS + warp;
-  if (t >= tokens) return;
-  const T* row = h + static_cast<size_t>(t) * d;
-
-  float ss = 0.f;
-  for (int j = lane * 8; j < d; j += 256) {
-    float v[8];
-    load8<T>(row + j, v);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  const float rstd = 1.0f / sqrtf(ss / static_cast<float>(d) + eps);
-
-  for (int e0 = 0; e0 < E; e0 += 8) {
-    float acc[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (int j = lane * 8; j < d; j += 256) {
-      float v[8], w[8];
-      load8<T>(row + j, v);
-      load8<float>(norm_w + j, w);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = w[i] * (v[i] * rstd);
-      if (e0 == 0) {
-        uint32_t packed[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          packed[i] = h2_as_u32(__halves2half2(to_half_sat(v[2 * i]), to_half_sat(v[2 * i + 1])));
-        *reinterpret_cast<uint4*>(xn_out + static_cast<size_t>(t) * d + j) =
-            make_uint4(packed[0], packed[1], packed[2], packed[3]);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (e0 + e < E) {
-          float r[8];
-          load8<float>(rw + static_cast<size_t>(e0 + e) * d + j, r);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc[e] = fmaf(v[i], r[i], acc[e]);
-        }
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-      if (lane == 0 && e0 + e < E) s_logit[warp][e0 + e] = acc[e] + (rb ? rb[e0 + e] : 0.f);
-    }
-  }
-  __syncwarp();
-
-  // softmax over E <= 64: lane owns experts lane and lane+32
-  const float NEG = -INFINITY;
-  float l0 = lane < E ? s_logit[warp][lane] : NEG;
-  float l1 = lane + 32 < E ? s_logit[warp][lane + 32] : NEG;
-  float mx = fmaxf(l0, l1);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float p0 = lane < E ? expf(l0 - mx) : 0.f;
-  float p1 = lane + 32 < E ? expf(l1 - mx) : 0.f;
-  float sum = p0 + p1;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  p0 = lane < E ? p0 / sum : -1.f;
-  p1 = lane + 32 < E ? p1 / sum : -1.f;
-
-  float sel_p[MAX_TOPK];
-  int sel_i[MAX_TOPK];
-  float gsum = 0.f;
-#pragma unroll
-  for (int i = 0; i < MAX_TOPK; ++i) {
-    if (i < k) {
-      float bp = p0;
-      int bi = lane;
-      if (p1 > bp) { bp = p1; bi = lane + 32; }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float op = __shfl_xor_sync(0xffffffffu, bp, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (op > bp || (op == bp && oi < bi)) { bp = op; bi = oi; }
-      }
-      sel_p[i] = bp;
-      sel_i[i] = bi;
-      gsum += bp;
-      if (bi == lane) p0 = -1.f;
-      if (bi == lane + 32) p1 = -1.f;
-    }
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < MAX_TOPK; ++i) {
-      if (i < k) {
-        experts_out[static_cast<size_t>(t) * k + i] = sel_i[i];
-        gates_out[static_cast<size_t>(t) * k + i] = sel_p[i] / gsum;
-      }
-    }
-  }
-}
-
 // Softmax over the logits of one token held in shared memory, top-k and gate
-// renormalisation by one warp (shared by both router kernels).
+// renormalisation by one warp (shared by the router kernels).
 __device__ __forceinline__ void router_select(const float* logit, int lane, int E, int k,
                                               int32_t* experts_out, float* gates_out) {
   const float NEG = -INFINITY;
@@ -196,227 +87,227 @@ __device__ __forceinline__ void router_select(const float* logit, int lane, int 
   }
 }
 
-// Prefill: persistent CTAs with the router weight and the norm weight resident
-// in shared memory.  With one token per warp reading them from global memory,
-// every warp streams the whole router weight (E x d fp32) out of L2 for itself:
-// 4096 tokens x 128 KB for a Mixtral layer, which is what that kernel's time is.
-// Here a CTA loads them once (E*d*4 + d*4 bytes, up to ~220 KB) and its eight
-// warps walk over the tokens; only the activations move through HBM.  Per token
-// the operations and their order are those of router_kernel, so experts and gates
-// are bit-identical to it.
-//
-// Shared layout: element j = 256*it + 8*lane + 4*hf + i of a vector is stored at
-// ((it*2 + hf)*32 + lane)*4 + i, so that the two 16-byte reads a lane makes per
-// step are conflict-free.
-constexpr int RS_WARPS = 8;
+// Many tokens: one CTA routes RT_TOKENS tokens at a time, warp w taking the column
+// chunks w, w + 8, ... of 256.  Every router weight that is loaded serves four tokens,
+// and the CTAs of an SM share the weights through L1; the kernel before this one (a
+// warp per token, weights in shared memory, one 8-warp CTA per SM) waited for latency
+// most of the time.  Writes the token's rstd and the CTA's expert counts for
+// route_permute_kernel, or (xn_out) the normalised rows as fp16.
+// One B200, us: 4096 tokens, hidden 4096, 8 experts 59 -> RT_A; 8192 tokens, hidden 6144
+// 186 -> RT_B; 777 tokens 42 -> RT_C.
+constexpr int RT_TOKENS = 4;
+constexpr int RT_THREADS = 256;
 
 template <typename T>
-__global__ void __launch_bounds__(RS_WARPS * 32)
-router_smem_kernel(const T* __restrict__ h, int tokens, int d, int E, int k, float eps,
-                   const float* __restrict__ norm_w, const float* __restrict__ rw,
-                   const float* __restrict__ rb, __half* __restrict__ xn_out,
-                   int32_t* __restrict__ experts_out, float* __restrict__ gates_out) {
-  extern __shared__ float s_dyn[];
-  float* s_w = s_dyn;                       // [E][d] in the layout above
-  float* s_n = s_dyn + static_cast<size_t>(E) * d;  // [d]
-  float* s_logit = s_n + d;                 // [RS_WARPS][MAX_EXPERTS]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto slot = [](int j) { return (((j >> 8) * 2 + ((j >> 2) & 1)) * 32 + ((j >> 3) & 31)) * 4 + (j & 3); };
-  for (int idx = threadIdx.x * 4; idx < E * d; idx += RS_WARPS * 32 * 4) {
-    const int e = idx / d, j = idx - e * d;
-    *reinterpret_cast<float4*>(s_w + static_cast<size_t>(e) * d + slot(j)) =
-        *reinterpret_cast<const float4*>(rw + idx);
-  }
-  for (int j = threadIdx.x * 4; j < d; j += RS_WARPS * 32 * 4)
-    *reinterpret_cast<float4*>(s_n + slot(j)) = *reinterpret_cast<const float4*>(norm_w + j);
-  __syncthreads();
-
-  for (int t = blockIdx.x * RS_WARPS + warp; t < tokens; t += gridDim.x * RS_WARPS) {
-    const T* row = h + static_cast<size_t>(t) * d;
-    float ss = 0.f;
-    for (int j = lane * 8; j < d; j += 256) {
-      float v[8];
-      load8<T>(row + j, v);
+__global__ void __launch_bounds__(RT_THREADS, 2)
+router_tokens_kernel(const T* __restrict__ h, int tokens, int d, int E, int k, float eps,
+                     const float* __restrict__ norm_w, const float* __restrict__ rw,
+                     const float* __restrict__ rb, __half* __restrict__ xn_out,
+                     int32_t* __restrict__ experts_out, float* __restrict__ gates_out,
+                     float* __restrict__ rstd_out, int32_t* __restrict__ hist) {
+  constexpr int WARPS = RT_THREADS / 32;
+  __shared__ float s_part[WARPS][RT_TOKENS][9];  // eight logit sums, sum of squares
+  __shared__ float s_logit[RT_TOKENS][MAX_EXPERTS];
+  __shared__ float s_rstd[RT_TOKENS];
+  __shared__ int32_t s_sel[RT_TOKENS * MAX_TOPK];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int t0 = blockIdx.x * RT_TOKENS;
+  const int nt = min(RT_TOKENS, tokens - t0);
+  const T* rows = h + static_cast<size_t>(t0) * d;
+  for (int e0 = 0; e0 < E; e0 += 8) {
+    float acc[RT_TOKENS][9];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
-    }
+    for (int q = 0; q < RT_TOKENS; ++q)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rstd = 1.0f / sqrtf(ss / static_cast<float>(d) + eps);
-
-    for (int e0 = 0; e0 < E; e0 += 8) {
-      float acc[8];
+      for (int e = 0; e < 9; ++e) acc[q][e] = 0.f;
+    for (int j = warp * 256 + lane * 8; j < d; j += WARPS * 256) {
+      float x[RT_TOKENS][8], w[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-      for (int j = lane * 8; j < d; j += 256) {
-        float v[8], w[8];
-        load8<T>(row + j, v);  // second pass: the row is in L1/L2
-        const int base = ((j >> 8) * 2 * 32 + lane) * 4;  // hf = 0; hf = 1 is 128 floats further
-        {
-          const float4 a = *reinterpret_cast<const float4*>(s_n + base);
-          const float4 b = *reinterpret_cast<const float4*>(s_n + base + 128);
-          w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-          w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+      for (int q = 0; q < RT_TOKENS; ++q)
+        load8<T>(rows + static_cast<size_t>(q < nt ? q : 0) * d + j, x[q]);
+      load8<float>(norm_w + j, w);
+#pragma unroll
+      for (int q = 0; q < RT_TOKENS; ++q)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          acc[q][8] = fmaf(x[q][i], x[q][i], acc[q][8]);
+          x[q][i] *= w[i];
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = w[i] * (v[i] * rstd);
-        if (e0 == 0) {
-          uint32_t packed[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            packed[i] = h2_as_u32(__halves2half2(to_half_sat(v[2 * i]), to_half_sat(v[2 * i + 1])));
-          *reinterpret_cast<uint4*>(xn_out + static_cast<size_t>(t) * d + j) =
-              make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          if (e0 + e < E) {
-            const float* wr = s_w + static_cast<size_t>(e0 + e) * d + base;
-            const float4 a = *reinterpret_cast<const float4*>(wr);
-            const float4 b = *reinterpret_cast<const float4*>(wr + 128);
-            const float r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[e] = fmaf(v[i], r[i], acc[e]);
-          }
-        }
-      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
+        if (e0 + e < E) {
+          load8<float>(rw + static_cast<size_t>(e0 + e) * d + j, w);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-        if (lane == 0 && e0 + e < E)
-          s_logit[warp * MAX_EXPERTS + e0 + e] = acc[e] + (rb ? rb[e0 + e] : 0.f);
+          for (int q = 0; q < RT_TOKENS; ++q)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[q][e] = fmaf(x[q][i], w[i], acc[q][e]);
+        }
       }
     }
+#pragma unroll
+    for (int q = 0; q < RT_TOKENS; ++q)
+#pragma unroll
+      for (int e = 0; e < 9; ++e) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[q][e] += __shfl_xor_sync(0xffffffffu, acc[q][e], o);
+        if (lane == 0) s_part[warp][q][e] = acc[q][e];
+      }
+    __syncthreads();
+    if (tid < RT_TOKENS * 8) {
+      const int q = tid >> 3, e = tid & 7;
+      float tot = 0.f, v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        tot += s_part[w][q][8];
+        v += s_part[w][q][e];
+      }
+      const float rstd = 1.0f / sqrtf(tot / static_cast<float>(d) + eps);
+      if (e0 + e < E) s_logit[q][e0 + e] = v * rstd + (rb ? rb[e0 + e] : 0.f);
+      if (e == 0) s_rstd[q] = rstd;
+    }
+    __syncthreads();
+  }
+  if (warp < nt) {
+    router_select(s_logit[warp], lane, E, k, s_sel + warp * k, gates_out + static_cast<size_t>(t0 + warp) * k);
     __syncwarp();
-    router_select(s_logit + warp * MAX_EXPERTS, lane, E, k, experts_out + static_cast<size_t>(t) * k,
-                  gates_out + static_cast<size_t>(t) * k);
-    __syncwarp();  // the logits are rewritten for the warp's next token
+    if (lane < k) experts_out[static_cast<size_t>(t0 + warp) * k + lane] = s_sel[warp * k + lane];
+    if (lane == 0 && rstd_out != nullptr) rstd_out[t0 + warp] = s_rstd[warp];
+  }
+  if (hist != nullptr) {
+    __syncthreads();
+    for (int e = tid; e < E; e += RT_THREADS) {
+      int c = 0;
+      for (int i = 0; i < nt * k; ++i) c += s_sel[i] == e;
+      hist[static_cast<size_t>(blockIdx.x) * E + e] = c;
+    }
+  }
+  if (xn_out != nullptr) {
+    for (int q = 0; q < nt; ++q) {
+      const float rstd = s_rstd[q];
+      for (int j = tid * 8; j < d; j += RT_THREADS * 8) {
+        float x[8], w[8];
+        load8<T>(rows + static_cast<size_t>(q) * d + j, x);  // second pass: from L1 / L2
+        load8<float>(norm_w + j, w);
+        uint32_t packed[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          packed[i] = h2_as_u32(__halves2half2(to_half_sat(w[2 * i] * (x[2 * i] * rstd)),
+                                               to_half_sat(w[2 * i + 1] * (x[2 * i + 1] * rstd))));
+        *reinterpret_cast<uint4*>(xn_out + static_cast<size_t>(t0 + q) * d + j) =
+            make_uint4(packed[0], packed[1], packed[2], packed[3]);
+      }
+    }
   }
 }
 
-// The same kernel for bf16 activations with the token's row held in registers:
-// all of a row's loads are issued at once (one memory latency per token instead
-// of one per loop iteration) and, with PREFETCH, the next token's row is already
-// in flight while this one is being routed.  Arithmetic and its order are
-// unchanged.  MAXIT >= hidden / 256 (16: hidden up to 4096).
-template <int MAXIT, bool PREFETCH>
-__global__ void __launch_bounds__(RS_WARPS * 32)
-router_smem_bf16_kernel(const __nv_bfloat16* __restrict__ h, int tokens, int d, int E, int k, float eps,
-                        const float* __restrict__ norm_w, const float* __restrict__ rw,
-                        const float* __restrict__ rb, __half* __restrict__ xn_out,
-                        int32_t* __restrict__ experts_out, float* __restrict__ gates_out) {
-  extern __shared__ float s_dyn[];
-  float* s_w = s_dyn;
-  float* s_n = s_dyn + static_cast<size_t>(E) * d;
-  float* s_logit = s_n + d;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nit = d >> 8;
-  const int stride = gridDim.x * RS_WARPS;
-  int t = blockIdx.x * RS_WARPS + warp;
-  uint4 cur[MAXIT], nxt[PREFETCH ? MAXIT : 1];
-#define B200_LOAD_ROW(dst, tok)                                                              \
-  {                                                                                          \
-    const uint4* row_ = reinterpret_cast<const uint4*>(h + static_cast<size_t>(tok) * d) + lane; \
-    _Pragma("unroll") for (int it = 0; it < MAXIT; ++it) if (it < nit) dst[it] = row_[it * 32];  \
-  }
-  if (t < tokens) B200_LOAD_ROW(cur, t);  // in flight while the weights are staged
-  auto slot = [](int j) { return (((j >> 8) * 2 + ((j >> 2) & 1)) * 32 + ((j >> 3) & 31)) * 4 + (j & 3); };
-  for (int idx = threadIdx.x * 4; idx < E * d; idx += RS_WARPS * 32 * 4) {
-    const int e = idx / d, j = idx - e * d;
-    *reinterpret_cast<float4*>(s_w + static_cast<size_t>(e) * d + slot(j)) =
-        *reinterpret_cast<const float4*>(rw + idx);
-  }
-  for (int j = threadIdx.x * 4; j < d; j += RS_WARPS * 32 * 4)
-    *reinterpret_cast<float4*>(s_n + slot(j)) = *reinterpret_cast<const float4*>(norm_w + j);
+// Route plan, norm and row permutation of a whole prefill call, after
+// router_tokens_kernel: one CTA per RP_TOKENS tokens adds up the router CTAs' expert
+// counts (all of them for the segment offsets, those before it for its own rank base),
+// ranks its pairs (stable by pair index, as route_plan_kernel does) and writes each
+// token's normalised row to its k sorted positions.  The row is read once and never
+// stored unpermuted: plan and permutation took two launches and three passes over the
+// fp16 rows.  One B200, us, plan + permutation -> this kernel: 4096 tokens, hidden 4096,
+// top 2 11 + 17 -> RP_A; 8192 tokens, hidden 6144 20 + 56 -> RP_B.
+constexpr int RP_TOKENS = 16;
+constexpr int RP_THREADS = 256;
+// the counts are read whole by every CTA: up to 64 KB of them
+constexpr long long RP_MAX_COUNTS = 16384;
+
+template <typename T>
+__global__ void __launch_bounds__(RP_THREADS)
+route_permute_kernel(const T* __restrict__ h, int tokens, int d, int E, int k,
+                     const float* __restrict__ norm_w, const float* __restrict__ rstd,
+                     const int32_t* __restrict__ experts, const int32_t* __restrict__ hist,
+                     int32_t* __restrict__ counts, int32_t* __restrict__ seg, int32_t* __restrict__ perm,
+                     int32_t* __restrict__ inv, int kperm, uint4* __restrict__ xs) {
+  __shared__ int s_total[MAX_EXPERTS], s_before[MAX_EXPERTS], s_seg[MAX_EXPERTS + 1];
+  __shared__ int s_e[RP_TOKENS * MAX_TOPK], s_pos[RP_TOKENS * MAX_TOPK];
+  static_assert(RP_TOKENS % RT_TOKENS == 0, "a CTA starts at a router CTA's first token");
+  const int tid = threadIdx.x;
+  const int t0 = blockIdx.x * RP_TOKENS;
+  const int nt = min(RP_TOKENS, tokens - t0);
+  const int np = nt * k;
+  grid_dep_wait();
+  grid_dep_launch();
+  for (int e = tid; e < MAX_EXPERTS; e += RP_THREADS) s_total[e] = s_before[e] = 0;
+  for (int i = tid; i < np; i += RP_THREADS) s_e[i] = experts[static_cast<size_t>(t0) * k + i];
   __syncthreads();
-
-  auto unpack = [](const uint4& raw, float (&v)[8]) {
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[2 * i] = __uint_as_float(w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  // consecutive threads take consecutive (count row, expert) entries; with a power-of-two
+  // E a thread stays on one expert and adds up in registers
+  const int rows = (tokens + RT_TOKENS - 1) / RT_TOKENS, mine = t0 / RT_TOKENS;
+  if (RP_THREADS % E == 0) {
+    const int e = tid % E;
+    int all = 0, before = 0;
+    for (int i = tid; i < rows * E; i += RP_THREADS) {
+      const int c = hist[i];
+      all += c;
+      if (i < mine * E) before += c;
     }
-  };
-
-  for (; t < tokens; t += stride) {
-    if constexpr (PREFETCH) {
-      if (t + stride < tokens) B200_LOAD_ROW(nxt, t + stride);
-    }
-    float ss = 0.f;
-#pragma unroll
-    for (int it = 0; it < MAXIT; ++it) {
-      if (it < nit) {
-        float v[8];
-        unpack(cur[it], v);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ss = fmaf(v[i], v[i], ss);
+    atomicAdd(&s_total[e], all);
+    atomicAdd(&s_before[e], before);
+  } else {
+    for (int i = tid; i < rows * E; i += RP_THREADS) {
+      const int c = hist[i], e = i % E;
+      if (c != 0) {
+        atomicAdd(&s_total[e], c);
+        if (i < mine * E) atomicAdd(&s_before[e], c);
       }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rstd = 1.0f / sqrtf(ss / static_cast<float>(d) + eps);
-
-    for (int e0 = 0; e0 < E; e0 += 8) {
-      float acc[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-#pragma unroll
-      for (int it = 0; it < MAXIT; ++it) {
-        if (it < nit) {
-          float v[8], w[8];
-          unpack(cur[it], v);
-          const int base = (it * 2 * 32 + lane) * 4;
-          {
-            const float4 a = *reinterpret_cast<const float4*>(s_n + base);
-            const float4 b = *reinterpret_cast<const float4*>(s_n + base + 128);
-            w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-            w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = w[i] * (v[i] * rstd);
-          if (e0 == 0) {
-            uint32_t packed[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              packed[i] = h2_as_u32(__halves2half2(to_half_sat(v[2 * i]), to_half_sat(v[2 * i + 1])));
-            *reinterpret_cast<uint4*>(xn_out + static_cast<size_t>(t) * d + it * 256 + lane * 8) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (e0 + e < E) {
-              const float* wr = s_w + static_cast<size_t>(e0 + e) * d + base;
-              const float4 a = *reinterpret_cast<const float4*>(wr);
-              const float4 b = *reinterpret_cast<const float4*>(wr + 128);
-              const float r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-              for (int i = 0; i < 8; ++i) acc[e] = fmaf(v[i], r[i], acc[e]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-        if (lane == 0 && e0 + e < E)
-          s_logit[warp * MAX_EXPERTS + e0 + e] = acc[e] + (rb ? rb[e0 + e] : 0.f);
-      }
-    }
-    __syncwarp();
-    router_select(s_logit + warp * MAX_EXPERTS, lane, E, k, experts_out + static_cast<size_t>(t) * k,
-                  gates_out + static_cast<size_t>(t) * k);
-    __syncwarp();
-    if constexpr (PREFETCH) {
-#pragma unroll
-      for (int it = 0; it < MAXIT; ++it) cur[it] = nxt[it];
-    } else {
-      if (t + stride < tokens) B200_LOAD_ROW(cur, t + stride);
     }
   }
-#undef B200_LOAD_ROW
+  __syncthreads();
+  if (tid == 0) {
+    int run = 0;
+    for (int e = 0; e < E; ++e) {
+      s_seg[e] = run;
+      run += s_total[e];
+    }
+    s_seg[E] = run;
+  }
+  __syncthreads();
+  if (blockIdx.x == 0)
+    for (int e = tid; e <= E; e += RP_THREADS) {
+      seg[e] = s_seg[e];
+      if (e < E) counts[e] = s_total[e];
+    }
+  for (int i = tid; i < np; i += RP_THREADS) {
+    const int e = s_e[i];
+    int rank = 0;
+    for (int j = 0; j < i; ++j) rank += s_e[j] == e;
+    const int pos = s_seg[e] + s_before[e] + rank;
+    const int p = t0 * k + i;
+    s_pos[i] = pos;
+    perm[pos] = p;
+    inv[p] = pos;
+  }
+  __syncthreads();
+  const int warp = tid >> 5, lane = tid & 31;
+  const int nvec = d / 8;
+  for (int q = warp; q < nt; q += RP_THREADS / 32) {
+    const T* row = h + static_cast<size_t>(t0 + q) * d;
+    const float r = rstd[t0 + q];
+#pragma unroll 4
+    for (int j = lane; j < nvec; j += 32) {
+      float x[8], w[8];
+      load8<T>(row + j * 8, x);
+      load8<float>(norm_w + j * 8, w);
+      __half v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = to_half_sat(w[i] * (x[i] * r));
+      uint4 o;
+      if (kperm) {  // halves in the order 0,4,1,5,2,6,3,7 (see permute_rows_kernel)
+        o.x = h2_as_u32(__halves2half2(v[0], v[4]));
+        o.y = h2_as_u32(__halves2half2(v[1], v[5]));
+        o.z = h2_as_u32(__halves2half2(v[2], v[6]));
+        o.w = h2_as_u32(__halves2half2(v[3], v[7]));
+      } else {
+        o.x = h2_as_u32(__halves2half2(v[0], v[1]));
+        o.y = h2_as_u32(__halves2half2(v[2], v[3]));
+        o.z = h2_as_u32(__halves2half2(v[4], v[5]));
+        o.w = h2_as_u32(__halves2half2(v[6], v[7]));
+      }
+      for (int s = 0; s < k; ++s) xs[static_cast<size_t>(s_pos[q * k + s]) * nvec + j] = o;
+    }
+  }
 }
 
 // One CTA per token: used for small token counts (decode), where a warp per
@@ -766,49 +657,56 @@ int launch_router(const void* h, int h_dtype, int tokens, const b200moe_layer_t*
     B200_CHECK_CUDA(cudaGetLastError());
     return B200MOE_OK;
   }
-  const size_t rs_smem = (static_cast<size_t>(L->experts) * L->hidden + L->hidden +
-                          RS_WARPS * MAX_EXPERTS) * sizeof(float);
-  if (tokens >= 1024 && rs_smem <= 227 * 1024) {
-    const int ctas = min(sm_count(), (tokens + RS_WARPS - 1) / RS_WARPS);
-    const void* fn;
-    int which;
-    if (h_dtype == B200MOE_DT_F32) {
-      fn = reinterpret_cast<const void*>(&router_smem_kernel<float>); which = 0;
-    } else if (L->hidden <= 4096) {
-      fn = reinterpret_cast<const void*>(&router_smem_bf16_kernel<16, true>); which = 1;
-    } else {  // longer rows do not fit the register file twice over: two passes over global memory
-      fn = reinterpret_cast<const void*>(&router_smem_kernel<__nv_bfloat16>); which = 3;
-    }
-    static bool configured[16][4] = {};
-    int dev = 0;
-    B200_CHECK_CUDA(cudaGetDevice(&dev));
-    if (dev < 16 && !configured[dev][which]) {
-      B200_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-      configured[dev][which] = true;
-    }
-    int d_ = L->hidden, E_ = L->experts, k_ = L->top_k;
-    float eps_ = L->rms_epsilon;
-    const float *nw = L->ffn_norm_weight, *rwp = L->router_weight, *rbp = L->router_bias;
-    __half* xnp = static_cast<__half*>(xn);
-    void* args[] = {&h, &tokens, &d_, &E_, &k_, &eps_, &nw, &rwp, &rbp, &xnp, &experts, &gates};
-    B200_CHECK_CUDA(cudaLaunchKernel(fn, dim3(ctas), dim3(RS_WARPS * 32), args, rs_smem, st));
-    return B200MOE_OK;
-  }
-  dim3 grid((tokens + ROUTER_WARPS - 1) / ROUTER_WARPS), block(ROUTER_WARPS * 32);
-  if (h_dtype == B200MOE_DT_F32) {
-    router_kernel<float><<<grid, block, 0, st>>>(
+  const dim3 grid((tokens + RT_TOKENS - 1) / RT_TOKENS), block(RT_THREADS);
+  if (h_dtype == B200MOE_DT_F32)
+    router_tokens_kernel<float><<<grid, block, 0, st>>>(
         static_cast<const float*>(h), tokens, L->hidden, L->experts, L->top_k, L->rms_epsilon,
-        L->ffn_norm_weight, L->router_weight, L->router_bias, static_cast<__half*>(xn), experts,
-        gates);
-  } else if (h_dtype == B200MOE_DT_BF16) {
-    router_kernel<__nv_bfloat16><<<grid, block, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(h), tokens, L->hidden, L->experts, L->top_k,
-        L->rms_epsilon, L->ffn_norm_weight, L->router_weight, L->router_bias,
-        static_cast<__half*>(xn), experts, gates);
-  } else {
-    B200_REQUIRE(false, "router: activations must be fp32 or bf16");
-  }
+        L->ffn_norm_weight, L->router_weight, L->router_bias, static_cast<__half*>(xn), experts, gates, nullptr,
+        nullptr);
+  else
+    router_tokens_kernel<__nv_bfloat16><<<grid, block, 0, st>>>(
+        static_cast<const __nv_bfloat16*>(h), tokens, L->hidden, L->experts, L->top_k, L->rms_epsilon,
+        L->ffn_norm_weight, L->router_weight, L->router_bias, static_cast<__half*>(xn), experts, gates, nullptr,
+        nullptr);
   B200_CHECK_CUDA(cudaGetLastError());
+  return B200MOE_OK;
+}
+
+// Above the fused front's token count, while the count rows stay small enough to be
+// read whole by every CTA of the second kernel.
+bool front_prefill_supported(int tokens, const b200moe_layer_t* L) {
+  return tokens > FRONT_MAX_TOKENS && L->hidden % 256 == 0 && L->experts >= 1 && L->experts <= MAX_EXPERTS &&
+         L->top_k >= 1 && L->top_k <= MAX_TOPK && L->top_k <= L->experts &&
+         static_cast<long long>((tokens + RT_TOKENS - 1) / RT_TOKENS) * L->experts <= RP_MAX_COUNTS;
+}
+
+// Router, plan and permutation of a prefill call in two launches.  `scratch` holds
+// tokens floats and the count rows; the caller's fp16 row buffer (tokens * hidden * 2
+// bytes, not written on this path) is large enough.
+int launch_front_prefill(const void* h, int h_dtype, int tokens, const b200moe_layer_t* L, int32_t* experts,
+                         float* gates, int32_t* counts, int32_t* seg, int32_t* perm, int32_t* inv, int kperm,
+                         void* xs, void* scratch, cudaStream_t st) {
+  B200_REQUIRE(front_prefill_supported(tokens, L), "front: unsupported shape (tokens %d, hidden %d, experts %d)",
+               tokens, L->hidden, L->experts);
+  B200_REQUIRE(h_dtype == B200MOE_DT_F32 || h_dtype == B200MOE_DT_BF16, "front: activations must be fp32 or bf16");
+  float* rstd = static_cast<float*>(scratch);
+  int32_t* hist = reinterpret_cast<int32_t*>(rstd + tokens);
+  const dim3 rgrid((tokens + RT_TOKENS - 1) / RT_TOKENS), pgrid((tokens + RP_TOKENS - 1) / RP_TOKENS);
+#define B200_FRONT(T)                                                                                              \
+  router_tokens_kernel<T><<<rgrid, RT_THREADS, 0, st>>>(                                                           \
+      static_cast<const T*>(h), tokens, L->hidden, L->experts, L->top_k, L->rms_epsilon, L->ffn_norm_weight,       \
+      L->router_weight, L->router_bias, nullptr, experts, gates, rstd, hist);                                      \
+  B200_CHECK_CUDA(cudaGetLastError());                                                                             \
+  B200_CHECK_CUDA(launch_dependent(route_permute_kernel<T>, pgrid, dim3(RP_THREADS), 0, st,                        \
+                                   static_cast<const T*>(h), tokens, L->hidden, L->experts, L->top_k,              \
+                                   L->ffn_norm_weight, rstd, experts, hist, counts, seg, perm, inv, kperm,         \
+                                   static_cast<uint4*>(xs)));
+  if (h_dtype == B200MOE_DT_F32) {
+    B200_FRONT(float)
+  } else {
+    B200_FRONT(__nv_bfloat16)
+  }
+#undef B200_FRONT
   return B200MOE_OK;
 }
 
