@@ -87,14 +87,37 @@ __device__ __forceinline__ void router_select(const float* logit, int lane, int 
   }
 }
 
+// Sums of eight values over the warp: after each of the first three exchanges a lane
+// keeps half of the values, so 9 shuffles do what eight butterflies do in 40, with the
+// additions of a plain xor-16-8-4-2-1 butterfly.  Returns, on every lane, the sum of
+// value 4*bit4 + 2*bit3 + bit2 of the lane number.
+__device__ __forceinline__ float warp_sum8(const float (&a)[9], int lane) {
+  float b[4], c[2];
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b[i] = (h4 ? a[4 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, h4 ? a[i] : a[4 + i], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) c[i] = (h3 ? b[2 + i] : b[i]) + __shfl_xor_sync(0xffffffffu, h3 ? b[i] : b[2 + i], 8);
+  float v = (h2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, h2 ? c[0] : c[1], 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
+}
+__device__ __forceinline__ int warp_sum8_index(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // Many tokens: one CTA routes RT_TOKENS tokens at a time, warp w taking the column
 // chunks w, w + 8, ... of 256.  Every router weight that is loaded serves four tokens,
 // and the CTAs of an SM share the weights through L1; the kernel before this one (a
 // warp per token, weights in shared memory, one 8-warp CTA per SM) waited for latency
 // most of the time.  Writes the token's rstd and the CTA's expert counts for
 // route_permute_kernel, or (xn_out) the normalised rows as fp16.
-// One B200, us: 4096 tokens, hidden 4096, 8 experts 59 -> RT_A; 8192 tokens, hidden 6144
-// 186 -> RT_B; 777 tokens 42 -> RT_C.
+// One B200, us: 4096 tokens, hidden 4096, 8 experts 59 -> 35; 8192 tokens, hidden 6144
+// 186 -> 78; 777 tokens 42 -> 14.
 constexpr int RT_TOKENS = 4;
 constexpr int RT_THREADS = 256;
 
@@ -145,13 +168,11 @@ router_tokens_kernel(const T* __restrict__ h, int tokens, int d, int E, int k, f
       }
     }
 #pragma unroll
-    for (int q = 0; q < RT_TOKENS; ++q)
-#pragma unroll
-      for (int e = 0; e < 9; ++e) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[q][e] += __shfl_xor_sync(0xffffffffu, acc[q][e], o);
-        if (lane == 0) s_part[warp][q][e] = acc[q][e];
-      }
+    for (int q = 0; q < RT_TOKENS; ++q) {
+      const float v = warp_sum8(acc[q], lane), ss = warp_sum(acc[q][8]);
+      if ((lane & 3) == 0) s_part[warp][q][warp_sum8_index(lane)] = v;
+      if (lane == 0) s_part[warp][q][8] = ss;
+    }
     __syncthreads();
     if (tid < RT_TOKENS * 8) {
       const int q = tid >> 3, e = tid & 7;
@@ -207,8 +228,8 @@ router_tokens_kernel(const T* __restrict__ h, int tokens, int d, int E, int k, f
 // token's normalised row to its k sorted positions.  The row is read once and never
 // stored unpermuted: plan and permutation took two launches and three passes over the
 // fp16 rows.  One B200, us, plan + permutation -> this kernel: 4096 tokens, hidden 4096,
-// top 2 11 + 17 -> RP_A; 8192 tokens, hidden 6144 20 + 56 -> RP_B.
-constexpr int RP_TOKENS = 16;
+// top 2 11 + 17 -> 21; 8192 tokens, hidden 6144 20 + 56 -> 61.
+constexpr int RP_TOKENS = 8;
 constexpr int RP_THREADS = 256;
 // the counts are read whole by every CTA: up to 64 KB of them
 constexpr long long RP_MAX_COUNTS = 16384;
@@ -232,19 +253,32 @@ route_permute_kernel(const T* __restrict__ h, int tokens, int d, int E, int k,
   for (int e = tid; e < MAX_EXPERTS; e += RP_THREADS) s_total[e] = s_before[e] = 0;
   for (int i = tid; i < np; i += RP_THREADS) s_e[i] = experts[static_cast<size_t>(t0) * k + i];
   __syncthreads();
-  // consecutive threads take consecutive (count row, expert) entries; with a power-of-two
-  // E a thread stays on one expert and adds up in registers
+  // consecutive threads take consecutive (count row, expert) entries; where E divides
+  // the CTA's stride a thread stays on its four experts and adds up in registers
   const int rows = (tokens + RT_TOKENS - 1) / RT_TOKENS, mine = t0 / RT_TOKENS;
-  if (RP_THREADS % E == 0) {
-    const int e = tid % E;
-    int all = 0, before = 0;
-    for (int i = tid; i < rows * E; i += RP_THREADS) {
-      const int c = hist[i];
-      all += c;
-      if (i < mine * E) before += c;
+  if (E % 4 == 0 && (4 * RP_THREADS) % E == 0) {
+    const int4* h4 = reinterpret_cast<const int4*>(hist);
+    int4 all = make_int4(0, 0, 0, 0), before = all;
+#pragma unroll 8
+    for (int i = tid; i < rows * E / 4; i += RP_THREADS) {
+      const int4 c = h4[i];
+      all.x += c.x; all.y += c.y; all.z += c.z; all.w += c.w;
+      if (4 * i < mine * E) { before.x += c.x; before.y += c.y; before.z += c.z; before.w += c.w; }
     }
-    atomicAdd(&s_total[e], all);
-    atomicAdd(&s_before[e], before);
+    const int e = (4 * tid) % E;
+    // lanes E/4 apart hold the same experts
+    for (int o = 16; o >= E / 4 && o > 0; o >>= 1) {
+      all.x += __shfl_xor_sync(0xffffffffu, all.x, o); all.y += __shfl_xor_sync(0xffffffffu, all.y, o);
+      all.z += __shfl_xor_sync(0xffffffffu, all.z, o); all.w += __shfl_xor_sync(0xffffffffu, all.w, o);
+      before.x += __shfl_xor_sync(0xffffffffu, before.x, o); before.y += __shfl_xor_sync(0xffffffffu, before.y, o);
+      before.z += __shfl_xor_sync(0xffffffffu, before.z, o); before.w += __shfl_xor_sync(0xffffffffu, before.w, o);
+    }
+    if ((tid & 31) < E / 4) {
+      atomicAdd(&s_total[e], all.x); atomicAdd(&s_total[e + 1], all.y);
+      atomicAdd(&s_total[e + 2], all.z); atomicAdd(&s_total[e + 3], all.w);
+      atomicAdd(&s_before[e], before.x); atomicAdd(&s_before[e + 1], before.y);
+      atomicAdd(&s_before[e + 2], before.z); atomicAdd(&s_before[e + 3], before.w);
+    }
   } else {
     for (int i = tid; i < rows * E; i += RP_THREADS) {
       const int c = hist[i], e = i % E;
@@ -285,27 +319,35 @@ route_permute_kernel(const T* __restrict__ h, int tokens, int d, int E, int k,
   for (int q = warp; q < nt; q += RP_THREADS / 32) {
     const T* row = h + static_cast<size_t>(t0 + q) * d;
     const float r = rstd[t0 + q];
-#pragma unroll 4
-    for (int j = lane; j < nvec; j += 32) {
-      float x[8], w[8];
-      load8<T>(row + j * 8, x);
-      load8<float>(norm_w + j * 8, w);
-      __half v[8];
+    // four vectors at a time: their loads are in flight together (nvec is a multiple of 32)
+    for (int j0 = lane; j0 < nvec; j0 += 128) {
+      float x[4][8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = to_half_sat(w[i] * (x[i] * r));
-      uint4 o;
-      if (kperm) {  // halves in the order 0,4,1,5,2,6,3,7 (see permute_rows_kernel)
-        o.x = h2_as_u32(__halves2half2(v[0], v[4]));
-        o.y = h2_as_u32(__halves2half2(v[1], v[5]));
-        o.z = h2_as_u32(__halves2half2(v[2], v[6]));
-        o.w = h2_as_u32(__halves2half2(v[3], v[7]));
-      } else {
-        o.x = h2_as_u32(__halves2half2(v[0], v[1]));
-        o.y = h2_as_u32(__halves2half2(v[2], v[3]));
-        o.z = h2_as_u32(__halves2half2(v[4], v[5]));
-        o.w = h2_as_u32(__halves2half2(v[6], v[7]));
+      for (int u = 0; u < 4; ++u)
+        if (j0 + 32 * u < nvec) load8<T>(row + (j0 + 32 * u) * 8, x[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + 32 * u;
+        if (j >= nvec) break;
+        float w[8];
+        load8<float>(norm_w + j * 8, w);
+        __half v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = to_half_sat(w[i] * (x[u][i] * r));
+        uint4 o;
+        if (kperm) {  // halves in the order 0,4,1,5,2,6,3,7 (see permute_rows_kernel)
+          o.x = h2_as_u32(__halves2half2(v[0], v[4]));
+          o.y = h2_as_u32(__halves2half2(v[1], v[5]));
+          o.z = h2_as_u32(__halves2half2(v[2], v[6]));
+          o.w = h2_as_u32(__halves2half2(v[3], v[7]));
+        } else {
+          o.x = h2_as_u32(__halves2half2(v[0], v[1]));
+          o.y = h2_as_u32(__halves2half2(v[2], v[3]));
+          o.z = h2_as_u32(__halves2half2(v[4], v[5]));
+          o.w = h2_as_u32(__halves2half2(v[6], v[7]));
+        }
+        for (int s = 0; s < k; ++s) xs[static_cast<size_t>(s_pos[q * k + s]) * nvec + j] = o;
       }
-      for (int s = 0; s < k; ++s) xs[static_cast<size_t>(s_pos[q * k + s]) * nvec + j] = o;
     }
   }
 }
@@ -365,11 +407,10 @@ __device__ __forceinline__ void router_block_body(const T* __restrict__ row, int
         }
       }
     }
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
-      if (lane == 0) s_part[warp][e] = acc[e];
+    {
+      const float v = warp_sum8(acc, lane), ss = warp_sum(acc[8]);
+      if ((lane & 3) == 0) s_part[warp][warp_sum8_index(lane)] = v;
+      if (lane == 0) s_part[warp][8] = ss;
     }
     if (e0 == 0) loaded();
     __syncthreads();
@@ -690,7 +731,7 @@ int launch_front_prefill(const void* h, int h_dtype, int tokens, const b200moe_l
                tokens, L->hidden, L->experts);
   B200_REQUIRE(h_dtype == B200MOE_DT_F32 || h_dtype == B200MOE_DT_BF16, "front: activations must be fp32 or bf16");
   float* rstd = static_cast<float*>(scratch);
-  int32_t* hist = reinterpret_cast<int32_t*>(rstd + tokens);
+  int32_t* hist = reinterpret_cast<int32_t*>(rstd + (tokens + 3) / 4 * 4);  // read 16 bytes at a time
   const dim3 rgrid((tokens + RT_TOKENS - 1) / RT_TOKENS), pgrid((tokens + RP_TOKENS - 1) / RP_TOKENS);
 #define B200_FRONT(T)                                                                                              \
   router_tokens_kernel<T><<<rgrid, RT_THREADS, 0, st>>>(                                                           \
