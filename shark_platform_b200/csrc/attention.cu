@@ -105,6 +105,8 @@ __device__ __forceinline__ uint4 rope_rotate8<__half2>(uint4 raw, const float2* 
 template <bool VEC>
 __global__ void __launch_bounds__(128) rope_kv_write_kernel(const RopeArgs a) {
   __shared__ float2 s_cs[ROPE_CACHE];
+  grid_dep_wait();
+  grid_dep_launch();
   const int t = blockIdx.x;
   const int b = t / a.tokens_per_seq;
   const int pos = a.positions[t];
@@ -470,12 +472,19 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_kernel(const DecodeArg
 // O[head][d] = sum_pos P[head][pos] V[pos][d].  The accumulator fragment of S is,
 // element for element, the A fragment of P for the second product, so the
 // probabilities never leave registers.  Four warps per CTA; per stage of 64
-// positions every warp owns 16 of them with its own online-softmax state; the K
-// and V rows of a stage arrive by cp.async (16 bytes per lane, coalesced, rows
-// beyond the sequence zero-filled) into a two-stage ring, rows padded by 16 bytes
-// so that ldmatrix reads are conflict-free.  Per 16 positions a warp issues 32
+// positions every warp owns 16 of them, with its own online-softmax state and its own
+// two-slot ring of K and V rows: no block-wide barrier inside the loop, so a warp
+// that waits for memory holds up nobody else, and the page ids of the stage after the
+// next are read one stage ahead of the copies that need them.  Rows arrive by cp.async
+// (16 bytes per lane, coalesced, rows beyond the sequence zero-filled), padded by 16
+// bytes so that ldmatrix reads are conflict-free.  Per 16 positions a warp issues 32
 // MMAs and 16 ldmatrix for 8 KB of cache: the kernel is left to wait for memory.
+// Kernel and merge on one B200, us, with a ring shared by the block (two barriers per
+// stage) -> now: 32 sequences of 2048..4096 positions (403 MB) 82 -> 76, 8 x 2048
+// 21 -> 18, 1 x 8192 25 -> 18.  Three slots (two CTAs per SM instead of three): 86, 25, 23.
 constexpr int ADT_STAGE_POS = 64;
+constexpr int ADT_WARPS = AD_THREADS / 32;
+constexpr int ADT_WPOS = ADT_STAGE_POS / ADT_WARPS;  // 16 positions per warp and stage
 constexpr int ADT_STAGES = 2;
 
 template <typename TC>
@@ -525,10 +534,11 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
   constexpr int ROW_B = HD * 2;
   constexpr int ROW_PAD = ROW_B + 16;
   constexpr int CHUNKS = ROW_B / 16;
-  constexpr int TILE = ADT_STAGE_POS * ROW_PAD;       // one K or V tile of a stage
+  constexpr int TILE = ADT_WPOS * ROW_PAD;            // one warp's K or V rows of a stage
   constexpr int KSTEPS = HD / 16, DTILES = HD / 8;
-  extern __shared__ __align__(16) uint8_t s_ring[];   // [stage][K tile | V tile]
-  __shared__ long long s_row[ADT_STAGES][ADT_STAGE_POS];
+  extern __shared__ __align__(16) uint8_t s_ring[];   // [warp][slot][K rows | V rows]
+  grid_dep_wait();
+  grid_dep_launch();
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int gid = lane >> 2, tig = lane & 3;
@@ -562,34 +572,35 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
     qa2[s] = Mma16<TC>::pack(v[2], v[3]);
   }
 
-  auto issue_stage = [&](int st_i) {
-    const int slot = st_i % ADT_STAGES;
-    const int p0 = p_begin + st_i * ADT_STAGE_POS;
-    if (t < ADT_STAGE_POS) {
-      const int pos = p0 + t;
-      long long row = -1;
-      if (pos < p_end) {
-        const int pslot = pos / a.stride;
-        const long long page = pslot < a.pages_per_seq ? a.page_ids[b * a.pages_per_seq + pslot] : -1;
-        if (page < 0 || page >= a.page_count) {
-          atomicOr(a.status, DEV_ERR_BOUNDS);
-        } else {
-          row = static_cast<long long>(static_cast<size_t>(page) * page_elems +
-                                       ((static_cast<size_t>(a.block_index) * 2) * a.stride + pos % a.stride) * row_elems +
-                                       static_cast<size_t>(kvh) * HD);
-        }
-      }
-      s_row[slot][t] = row;
+  // element offset of the K row of this lane's position in stage st_i (lanes 0..15), -1 = none
+  auto row_of = [&](int st_i) -> long long {
+    const int pos = p_begin + st_i * ADT_STAGE_POS + warp * ADT_WPOS + lane;
+    if (lane >= ADT_WPOS || pos >= p_end) return -1;
+    const int pslot = pos / a.stride;
+    const long long page = pslot < a.pages_per_seq ? a.page_ids[b * a.pages_per_seq + pslot] : -1;
+    if (page < 0 || page >= a.page_count) {
+      atomicOr(a.status, DEV_ERR_BOUNDS);
+      return -1;
     }
-    __syncthreads();
-    uint8_t* kt = s_ring + slot * 2 * TILE;
-    uint8_t* vt = kt + TILE;
-    for (int i = t; i < ADT_STAGE_POS * CHUNKS; i += AD_THREADS) {
-      const int r = i / CHUNKS, c = i % CHUNKS;
-      const long long row = s_row[slot][r];
-      const TC* src = slab + (row >= 0 ? row : 0) + c * 8;
-      cp_async16_zfill(smem_u32(kt + r * ROW_PAD + c * 16), src, row >= 0);
-      cp_async16_zfill(smem_u32(vt + r * ROW_PAD + c * 16), src + v_off, row >= 0);
+    return static_cast<long long>(static_cast<size_t>(page) * page_elems +
+                                  ((static_cast<size_t>(a.block_index) * 2) * a.stride + pos % a.stride) * row_elems +
+                                  static_cast<size_t>(kvh) * HD);
+  };
+  const uint32_t ring = smem_u32(s_ring) + warp * (ADT_STAGES * 2 * TILE);
+  // copies the warp's rows of a stage; one commit group per call, also past the end
+  auto issue_stage = [&](int st_i, long long row) {
+    if (st_i < nstages) {
+      const uint32_t kt = ring + (st_i % ADT_STAGES) * 2 * TILE;
+      constexpr int RPI = 32 / CHUNKS;  // rows per pass of the warp
+      const int r0 = lane / CHUNKS, c = lane % CHUNKS;
+#pragma unroll
+      for (int i = 0; i < ADT_WPOS / RPI; ++i) {
+        const int r = i * RPI + r0;
+        const long long off = __shfl_sync(0xffffffffu, row, r);
+        const TC* src = slab + (off >= 0 ? off : 0) + c * 8;
+        cp_async16_zfill(kt + r * ROW_PAD + c * 16, src, off >= 0);
+        cp_async16_zfill(kt + TILE + r * ROW_PAD + c * 16, src + v_off, off >= 0);
+      }
     }
     cp_async_commit();
   };
@@ -599,19 +610,16 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
 #pragma unroll
   for (int j = 0; j < DTILES; ++j) o[j][0] = o[j][1] = 0.f;
 
-  if (nstages > 0) issue_stage(0);
+  for (int i = 0; i < ADT_STAGES - 1; ++i) issue_stage(i, row_of(i));
+  long long row_next = row_of(ADT_STAGES - 1);
   for (int st_i = 0; st_i < nstages; ++st_i) {
-    if (st_i + 1 < nstages) {
-      issue_stage(st_i + 1);   // its barrier also says: stage st_i - 1's slot is no longer read
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();           // stage st_i has landed for everyone
-    const int slot = st_i % ADT_STAGES;
-    const uint32_t kt = smem_u32(s_ring + slot * 2 * TILE) + warp * 16 * ROW_PAD;
+    issue_stage(st_i + ADT_STAGES - 1, row_next);  // into the slot of stage st_i - 1
+    row_next = row_of(st_i + ADT_STAGES);
+    cp_async_wait<ADT_STAGES - 1>();
+    __syncwarp();  // the warp's rows of stage st_i have landed
+    const uint32_t kt = ring + (st_i % ADT_STAGES) * 2 * TILE;
     const uint32_t vt = kt + TILE;
-    const int p0 = p_begin + st_i * ADT_STAGE_POS + warp * 16;  // this warp's 16 positions
+    const int p0 = p_begin + st_i * ADT_STAGE_POS + warp * ADT_WPOS;  // this warp's 16 positions
 
     // S[head][pos]: two n-tiles of 8 positions
     float sc[2][4];
@@ -674,6 +682,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
         o[j + 1][0] = c1[0]; o[j + 1][1] = c1[1];
       }
     }
+    __syncwarp();  // the slot is read: the next pass refills it
   }
   // this lane's share of the denominator -> the head's
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
@@ -721,6 +730,8 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
 __global__ void __launch_bounds__(128)
 attn_decode_merge_kernel(const float* __restrict__ partial, int splits, int G, int hd, int heads, int kv_heads,
                          void* __restrict__ out, int out_dtype) {
+  grid_dep_wait();
+  grid_dep_launch();
   const int head = blockIdx.x, b = blockIdx.y;
   const int kvh = head / G, g = head % G;
   const float* base = partial + ((static_cast<size_t>(b) * kv_heads + kvh) * splits) * G * (hd + 2) + g * (hd + 2);
@@ -743,21 +754,24 @@ attn_decode_merge_kernel(const float* __restrict__ partial, int splits, int G, i
 }
 
 int decode_splits(int bs, int kv_heads, int max_seq_len) {
-  // about six CTAs per SM (each holds 64-130 KB of shared-memory tiles at most
-  // three deep, and the steps of one CTA are serial), but no split shorter than
-  // one 128-position step
+  // Two to three CTAs of 128 positions per step or more are resident per SM; ragged
+  // lengths want somewhat more CTAs than that, every split costs the merge a partial
+  // result.  us on one B200 at 2 / 3 / 4 / 6 CTAs per SM asked for: 32 sequences of up
+  // to 4096 positions 85 / 86 / 82 / 87, 32 x 1024 33 / 33 / 31 / 34, 8 x 2048
+  // 24 / 21 / 24 / 25, 1 x 8192 (37 / 56 / 64 / 64 splits) 25 / 28 / 33 / 33.
   const int base = bs * kv_heads;
-  int splits = (6 * sm_count() + base - 1) / base;
+  const int per_sm = base >= sm_count() ? 4 : 3;
+  int splits = (per_sm * sm_count() + base - 1) / base;
   const int most = (max_seq_len + AD_THREADS - 1) / AD_THREADS;
   if (splits > most) splits = most;
   if (splits < 1) splits = 1;
-  if (splits > 64) splits = 64;
+  if (splits > 32) splits = 32;
   return splits;
 }
 
 template <typename TC, int HD>
 int launch_decode_mma(const DecodeArgs& a, dim3 grid, cudaStream_t st) {
-  constexpr int RING = ADT_STAGES * 2 * ADT_STAGE_POS * (HD * 2 + 16);
+  constexpr int RING = ADT_WARPS * ADT_STAGES * 2 * ADT_WPOS * (HD * 2 + 16);
   constexpr int MERGE = (4 * AD_MAXG * HD + 4 * AD_MAXG * 2) * 4;
   constexpr int SMEM = RING > MERGE ? RING : MERGE;
   auto kern = attn_decode_mma_kernel<TC, HD>;
@@ -768,8 +782,7 @@ int launch_decode_mma(const DecodeArgs& a, dim3 grid, cudaStream_t st) {
     B200_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     configured[dev] = true;
   }
-  kern<<<grid, AD_THREADS, SMEM, st>>>(a);
-  B200_CHECK_CUDA(cudaGetLastError());
+  B200_CHECK_CUDA(launch_dependent(kern, grid, dim3(AD_THREADS), SMEM, st, a));
   return B200MOE_OK;
 }
 
@@ -835,9 +848,10 @@ int b200moe_attn_rope_kv_write(void* q, const void* k, const void* v, void* k_ou
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = io_dtype == cache_dtype && io_dtype != B200MOE_DT_F32 && cache->head_dim % 8 == 0 &&
                    cache->head_dim / 2 <= ROPE_CACHE && al(q) && al(k) && al(v) && al(k_out) && al(v_out) && al(slab);
-  if (vec) rope_kv_write_kernel<true><<<tokens, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  else rope_kv_write_kernel<false><<<tokens, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
-  B200_CHECK_CUDA(cudaGetLastError());
+  if (vec)
+    B200_CHECK_CUDA(launch_dependent(rope_kv_write_kernel<true>, dim3(tokens), dim3(128), 0, static_cast<cudaStream_t>(stream), a));
+  else
+    B200_CHECK_CUDA(launch_dependent(rope_kv_write_kernel<false>, dim3(tokens), dim3(128), 0, static_cast<cudaStream_t>(stream), a));
   return B200MOE_OK;
 }
 
@@ -890,9 +904,8 @@ int b200moe_attn_decode(const void* q, int q_dtype, const void* slab, int cache_
     rc = hd == 64 ? launch_decode_mma<__nv_bfloat16, 64>(a, grid, st)
                   : launch_decode_mma<__nv_bfloat16, 128>(a, grid, st);
   if (rc) return rc;
-  attn_decode_merge_kernel<<<dim3(heads, bs), 128, 0, st>>>(a.partial, a.splits, heads / cache->kv_heads, hd, heads,
-                                                            cache->kv_heads, out, out_dtype);
-  B200_CHECK_CUDA(cudaGetLastError());
+  B200_CHECK_CUDA(launch_dependent(attn_decode_merge_kernel, dim3(heads, bs), dim3(128), 0, st, a.partial, a.splits,
+                                   heads / cache->kv_heads, hd, heads, cache->kv_heads, out, out_dtype));
   return B200MOE_OK;
 }
 
