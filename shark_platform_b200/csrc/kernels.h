@@ -63,7 +63,8 @@ int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile
 
 int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows);
 int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
-                     int ksplit, float* const* outs, cudaStream_t st);
+                     int ksplit, float* const* parts, void* const* outs, int out_dtype, const void* residual,
+                     cudaStream_t st);
 
 // the kernel AUTO takes for a product of `max_segment` rows at most (api.cu)
 int pick_regime(int regime, const b200moe_weight_t* w, int max_segment, bool down);

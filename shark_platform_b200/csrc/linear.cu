@@ -3,7 +3,7 @@
 //   1. linear_rows_kernel: the input rows as fp16 (optionally RMS-normalised first),
 //      in the column order(s) the weights' layouts read, plus the segment [0, rows];
 //   2. one launch for all weights of a layout (regime by the row count);
-//   3. linear_finish_kernel: the k-split partial sums of all outputs added, rounded
+//   3. where k was split, linear_finish_kernel: the k-split partial sums of all outputs added, rounded
 //      to the output type and, for a block's last projection, added to the residual.
 // Replaces, per linear, a cast, a column shuffle, a torch.tensor upload of the segment
 // (a host synchronisation), a sum over partials and a cast.  One B200, q/k/v/output
@@ -132,7 +132,7 @@ struct LinFinishArgs {
   long long n[LIN_MAX];         // rows * N (a multiple of 4)
   int ks[LIN_MAX];
   long long vec_end[LIN_MAX];   // running count of 4-element vectors
-  const void* residual;         // added to output 0, or NULL; output dtype
+  const void* residual;         // added to entry 0, or NULL; output dtype
   int count;
 };
 
@@ -205,6 +205,7 @@ struct LinGroup {
   int index[LIN_MAX];  // place in the caller's list
   int count, ks;
   bool tensor;
+  bool direct;  // the product writes the finished outputs itself
 };
 
 LinGroup lin_group(const b200moe_weight_t* const* w, int count, int rows, int layout) {
@@ -217,6 +218,7 @@ LinGroup lin_group(const b200moe_weight_t* const* w, int count, int rows, int la
     g.tensor = g.tensor && pick_regime(B200MOE_REGIME_AUTO, w[i], rows, true) == B200MOE_REGIME_TENSOR;
   }
   if (g.count > 0) g.ks = g.tensor ? tc_linear_ksplit(g.w, g.count, rows) : stream_linear_ksplit(g.w, g.count, rows);
+  g.direct = g.tensor && g.ks == 1;
   return g;
 }
 
@@ -227,7 +229,7 @@ struct LinWorkspace {
   __half* plain;
   __half* perm;
   float* part[LIN_MAX];
-  int ks[LIN_MAX];
+  int ks[LIN_MAX];  // 0: no partial sums
   size_t bytes;
 };
 
@@ -251,10 +253,10 @@ LinWorkspace lin_carve(const b200moe_weight_t* const* w, int count, int rows, bo
   if (perm) o.perm = static_cast<__half*>(take(row_bytes));
   for (int layout : LIN_LAYOUTS) {
     const LinGroup g = lin_group(w, count, rows, layout);
-    for (int i = 0; i < g.count; ++i) o.ks[g.index[i]] = g.ks;
+    for (int i = 0; i < g.count; ++i) o.ks[g.index[i]] = g.direct ? 0 : g.ks;
   }
   for (int i = 0; i < count; ++i)
-    o.part[i] = static_cast<float*>(take(static_cast<size_t>(o.ks[i]) * rows * w[i]->rows * 4));
+    if (o.ks[i] > 0) o.part[i] = static_cast<float*>(take(static_cast<size_t>(o.ks[i]) * rows * w[i]->rows * 4));
   o.bytes = off;
   return o;
 }
@@ -326,21 +328,28 @@ int b200moe_linear(const void* x, int x_dtype, int32_t rows, const float* norm_w
                      : x_ready                                        ? x
                                                                       : static_cast<const void*>(w.plain);
     float* parts[LIN_MAX] = {};
-    for (int i = 0; i < g.count; ++i) parts[i] = w.part[g.index[i]];
-    if (int rc = g.tensor ? launch_tc_linear(xs, w.seg, rows, g.w, g.count, g.ks, parts, st)
+    void* dst[LIN_MAX] = {};
+    for (int i = 0; i < g.count; ++i) {
+      parts[i] = w.part[g.index[i]];
+      dst[i] = outs[g.index[i]];
+    }
+    const void* res = g.index[0] == 0 ? residual : nullptr;
+    if (int rc = g.tensor ? launch_tc_linear(xs, w.seg, rows, g.w, g.count, g.ks, parts, dst, out_dtype, res, st)
                           : launch_stream_linear(xs, w.seg, rows, g.w, g.count, g.ks, parts, st))
       return rc;
   }
   for (int i = 0; i < count; ++i) {
-    fa.part[i] = w.part[i];
-    fa.out[i] = outs[i];
-    fa.ks[i] = w.ks[i];
-    fa.n[i] = static_cast<long long>(rows) * weights[i]->rows;
-    run += fa.n[i] / 4;
-    fa.vec_end[i] = run;
+    if (w.ks[i] == 0) continue;
+    const int o = fa.count++;
+    fa.part[o] = w.part[i];
+    fa.out[o] = outs[i];
+    fa.ks[o] = w.ks[i];
+    fa.n[o] = static_cast<long long>(rows) * weights[i]->rows;
+    run += fa.n[o] / 4;
+    fa.vec_end[o] = run;
+    if (i == 0) fa.residual = residual;
   }
-  fa.residual = residual;
-  fa.count = count;
+  if (fa.count == 0) return B200MOE_OK;
   const long long want = (run + 255) / 256, most = 16ll * sm_count();
   const unsigned ctas = static_cast<unsigned>(want < most ? want : most);
   if (out_dtype == B200MOE_DT_F32)

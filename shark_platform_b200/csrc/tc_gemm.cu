@@ -16,9 +16,9 @@
 //
 // Three independent shared-memory rings, because their slots live for very
 // different times:
-//   weights  2 slots x (2 sets x 128 rows x 128 k) int8, 128-byte swizzle;
+//   weights  2-5 slots x (2 sets x 128 rows x 128 k) int8, 128-byte swizzle;
 //            a slot is free again as soon as the dequant warps have read it
-//   tokens   6 slots x (192 rows x 64 k) fp16; a slot is held until the MMAs
+//   tokens   3 slots x (192 rows x 128 k) fp16; a slot is held until the MMAs
 //            that read it have completed
 //   scales   2 slots x (2 sets x 128 rows x 8) fp16 = 256 k
 //
@@ -27,6 +27,8 @@
 //               warps 4-7 set 1; warp w owns TMEM lanes 32(w%4)..+31), epilogue
 //   warps 8-15  group 1: the same for the odd stages, so that one group's
 //               tensor-memory store latency hides behind the other's arithmetic
+//               (the 64- and 128-token variants hand over two stages at a time:
+//               group g takes every second 128-k weight slot whole)
 //   warp  16    TMA producer for weights and scales
 //   warp  17    TMA producer for token tiles
 //   warp  18    TMEM allocation; issues the MMAs of row set 0 and commits
@@ -126,7 +128,32 @@ struct TcArgs {
   int mrows[3];
   float* mout[3];
   const uint8_t* mst[3];
+  // with an unsplit k the finished values go out at once: mdst[e] of type mdtype, the
+  // residual (of that type) added to matrix 0; else mout[e] gets fp32 partial sums
+  void* mdst[3];
+  int mdtype;
+  const void* residual;
 };
+
+__device__ __forceinline__ float tc_load_residual(const void* p, int dt, size_t i) {
+  if (dt == B200MOE_DT_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
+  if (dt == B200MOE_DT_F16) return __half2float(static_cast<const __half*>(p)[i]);
+  return static_cast<const float*>(p)[i];
+}
+// y rounded to its type and, with a residual, the sum rounded again (`h + y` on tensors).
+__device__ __forceinline__ void tc_store_linear(void* dst, int dt, bool add, float residual, size_t i, float v) {
+  if (dt == B200MOE_DT_BF16) {
+    __nv_bfloat16 r = __float2bfloat16_rn(v);
+    if (add) r = __float2bfloat16_rn(residual + __bfloat162float(r));
+    static_cast<__nv_bfloat16*>(dst)[i] = r;
+  } else if (dt == B200MOE_DT_F16) {
+    __half r = __float2half_rn(v);
+    if (add) r = __float2half_rn(residual + __half2float(r));
+    static_cast<__half*>(dst)[i] = r;
+  } else {
+    static_cast<float*>(dst)[i] = add ? residual + v : v;
+  }
+}
 
 __device__ __forceinline__ void tc_bulk_load(uint32_t dst, const void* src, uint32_t bytes,
                                              uint32_t bar) {
@@ -593,6 +620,40 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         float* obase = (MULTI ? args.mout[mat] : static_cast<float*>(args.out)) +
                        static_cast<size_t>((nt >> 16) & 0xff) * args.P * ostride +
                        static_cast<size_t>(row0) * ostride + (nt & 0xffff) * (2 * TC_ROWS) + row;
+        if (MULTI && args.ksplit == 1) {
+          void* const dst = args.mdst[mat];
+          const void* const res = mat == 0 ? args.residual : nullptr;
+          const size_t o0 = static_cast<size_t>(row0) * ostride + (nt & 0xffff) * (2 * TC_ROWS) + row;
+          for (int c0 = (grp * 2 + set) * 16; c0 < ncols; c0 += 64) {
+#pragma unroll 1
+            for (int h8 = 0; h8 < 16; h8 += 8) {
+              uint32_t g[8], u[8];
+              const int lim = rows - c0 - h8;
+              const size_t i0 = o0 + static_cast<size_t>(c0 + h8) * ostride;
+              // all residuals of the chunk before the first store: the compiler may not
+              // move a load above a store that could hit it, and one round trip per
+              // element made the drain twice as long as the products
+              float r0[8], r1[8];
+              if (res != nullptr) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  r0[j] = j < lim ? tc_load_residual(res, args.mdtype, i0 + j * ostride) : 0.f;
+                  r1[j] = j < lim ? tc_load_residual(res, args.mdtype, i0 + j * ostride + TC_ROWS) : 0.f;
+                }
+              }
+              tmem_ld8(tmem + lane_addr + TC_COL_ACC0 + c0 + h8, g);
+              tmem_ld8(tmem + lane_addr + TC_COL_ACC1 + c0 + h8, u);
+              tmem_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                if (j < lim) {
+                  tc_store_linear(dst, args.mdtype, res != nullptr, r0[j], i0 + j * ostride, __uint_as_float(g[j]));
+                  tc_store_linear(dst, args.mdtype, res != nullptr, r1[j], i0 + j * ostride + TC_ROWS, __uint_as_float(u[j]));
+                }
+              }
+            }
+          }
+        } else
         for (int c0 = (grp * 2 + set) * 16; c0 < ncols; c0 += 64) {
           uint32_t g[16], u[16];
           tmem_ld16(tmem + lane_addr + TC_COL_ACC0 + c0, g);
@@ -969,9 +1030,13 @@ int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows) {
   return best;
 }
 
-// outs[i] = fp32 [ksplit, rows, w[i]->rows] partial sums of xs w[i]^T; equal layouts and cols.
+// parts[i] = fp32 [ksplit, rows, w[i]->rows] partial sums of xs w[i]^T, or, with ksplit 1,
+// outs[i] = the products as out_dtype (residual added to outs[0]) and parts unused;
+// equal layouts and cols.  4096 rows of a 4096-wide block, one B200, us, product +
+// finish kernel -> now: q + k + v 157 + 44 -> 162, output with residual 112 + 39 -> 145.
 int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe_weight_t* const* w, int count,
-                     int ksplit, float* const* outs, cudaStream_t st) {
+                     int ksplit, float* const* parts, void* const* outs, int out_dtype, const void* residual,
+                     cudaStream_t st) {
   B200_REQUIRE(count >= 1 && count <= 3, "tensor kernel: 1..3 matrices");
   if (rows == 0) return B200MOE_OK;
   CUtensorMap maps[12] = {};
@@ -987,7 +1052,8 @@ int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe
     if (int rc = tc_weight_map(w[i], &maps[WMAP[i]], &maps[SMAP[i]])) return rc;
     a.mrows[i] = w[i]->rows;
     a.mtiles[i] = w[i]->rows / (2 * TC_ROWS);
-    a.mout[i] = outs[i];
+    a.mout[i] = parts[i];
+    a.mdst[i] = outs[i];
     a.mst[i] = static_cast<const uint8_t*>(w[i]->sub);
     row_tiles += a.mtiles[i];
     tiled_scales = tiled_scales && w[i]->sub != nullptr;
@@ -997,6 +1063,7 @@ int launch_tc_linear(const void* xs, const int32_t* seg, int rows, const b200moe
   if (int rc = tc_token_maps(maps, xs, rows, static_cast<uint64_t>(w[0]->cols) * 2)) return rc;
   B200_REQUIRE(ksplit >= 1 && (w[0]->cols / TC_KT) % (4 * ksplit) == 0, "tensor kernel: bad k split %d", ksplit);
   a.seg = seg; a.E = count; a.K = w[0]->cols; a.P = rows; a.ksplit = ksplit;
+  a.mdtype = out_dtype; a.residual = residual;
   a.row_tile = TC_ROWS;
   a.tok_tile = tc_linear_tok_tile(rows, row_tiles);
   a.status = device_status_ptr();
