@@ -41,3 +41,29 @@ def test_fewer_tokens_after_more_still_fit_the_workspace():
     for n in (1100, 512, 100, 3, 1):
         want = b200_block(case)(h[:n] if h.dim() == 2 else h.reshape(-1, 512)[:n])
         assert torch.equal(blk(h.reshape(-1, 512)[:n]), want)
+
+
+@pytest.mark.parametrize("tokens", [1, 40, 300])
+def test_captured_layer_call_equals_the_eager_one(tokens):
+    """The layer's kernels are launched as programmatic dependents: the same under capture."""
+    from shark_platform_b200 import moe
+
+    spec = syn.CaseSpec("graph", tokens, 512, 768, kind=syn.Q8_0, seed=73)
+    case = syn.make_case(spec)
+    blk = b200_block(case)
+    h = device_input(case).reshape(tokens, -1).contiguous()
+    want = blk(h)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        blk(h)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = blk(h)
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+    assert moe.device_status() == 0
