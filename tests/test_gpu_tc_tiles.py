@@ -67,3 +67,26 @@ def test_captured_layer_call_equals_the_eager_one(tokens):
         torch.cuda.synchronize()
         assert torch.equal(y, want)
     assert moe.device_status() == 0
+
+
+# 6 experts: the count rows are added up entry by entry; 129: one CTA past the decode
+# front; 515: a last router CTA of three tokens and a last permutation CTA of three
+@pytest.mark.parametrize("experts,top_k", [(4, 1), (6, 2), (16, 4), (64, 8)])
+@pytest.mark.parametrize("tokens", [129, 515])
+@pytest.mark.parametrize("act_dtype", ["bf16", "f32"])
+def test_prefill_front_routes_as_the_oracle(experts, top_k, tokens, act_dtype):
+    from shark_platform_b200 import moe
+
+    spec = syn.CaseSpec("front", tokens, 512, 256, experts, top_k, kind=syn.Q4_K if experts < 64 else syn.Q8_0,
+                        act_dtype=act_dtype, norm_weight="perturbed", router_bias="zipf", seed=74)
+    case = syn.make_case(spec)
+    y, ex, gates = b200_block(case).layer.forward(device_input(case), want_routing=True)
+    assert moe.device_status() == 0
+    want, mid = orc.moe_block(case.h, oracle_params(case), form="per_expert")
+    # a logit is an fp32 sum of 512 products of order one: off by about sqrt(512) * 2^-24
+    # = 1.3e-6, and so is a probability at most; tokens closer to a tie than 1e-5 are left out
+    p = torch.sort(mid["prob"], dim=-1, descending=True).values[:, : top_k + 1]
+    clear = (p[:, :-1] - p[:, 1:]).min(dim=1).values > 1e-5
+    assert clear.float().mean() > 0.9
+    assert torch.equal(ex.cpu().to(torch.int64)[clear], mid["experts"][clear])
+    assert orc.rel_l2(y.float().cpu().reshape(tokens, -1)[clear], want.reshape(tokens, -1)[clear]) < 2e-2
