@@ -127,12 +127,14 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 int g_token_tile = 192;
 
 // From this many tokens the tensor-memory kernel takes over from the
-// weight-streaming kernel (where the layout allows it).  One B200, Mixtral layer, us
-// per call, stream / tensor: Q8_0 16 tokens 278 / 292, 24 tokens 285 / 294, 32 tokens
-// 305 / 294, 64 tokens 366 / 309; Q4_K 16 tokens 261 / 267, 24 tokens 270 / 267,
-// 32 tokens 295 / 270.  A single matrix (attention projections): 4096 x 4096 Q8_0 24
-// rows 10.3 / 10.4, 32 rows 11.2 / 10.6, 64 rows 14.5 / 12.4.
+// weight-streaming kernel (where the layout allows it).  One B200, Mixtral layer,
+// gate/up + down, us, stream / tensor: Q8_0 16 tokens 262 / 276, 24 tokens 261 / 263,
+// 32 tokens 292 / 278, 64 tokens 344 / 289.  A single matrix (attention projections):
+// 4096 x 4096 Q8_0 24 rows 10.3 / 10.4, 32 rows 11.2 / 10.6, 64 rows 14.5 / 12.4.
+// Expert stacks of 4-bit weights change over earlier: 16 tokens 250 / 260, 24 tokens
+// 252 / 239 (hidden 2048, ffn 4096: 65 / 57; hidden 6144, ffn 16384: 419 / 395).
 constexpr int TENSOR_MIN_TOKENS = 32;
+constexpr int TENSOR_MIN_TOKENS_Q4 = 24;
 
 }  // namespace
 
@@ -144,8 +146,9 @@ int pick_regime(int regime, const b200moe_weight_t* w, int max_segment, bool dow
   if (regime == B200MOE_REGIME_TENSOR_PAIR) return B200MOE_REGIME_TENSOR_PAIR;
   if (regime == B200MOE_REGIME_STREAM) return B200MOE_REGIME_STREAM;
   const bool can_tensor = w != nullptr && tc_supported(w, down);
-  return (can_tensor && max_segment >= TENSOR_MIN_TOKENS) ? B200MOE_REGIME_TENSOR
-                                                          : B200MOE_REGIME_STREAM;
+  if (!can_tensor) return B200MOE_REGIME_STREAM;
+  const int least = w->layout == B200MOE_LAYOUT_Q4_K && w->experts >= 4 ? TENSOR_MIN_TOKENS_Q4 : TENSOR_MIN_TOKENS;
+  return max_segment >= least ? B200MOE_REGIME_TENSOR : B200MOE_REGIME_STREAM;
 }
 
 namespace {

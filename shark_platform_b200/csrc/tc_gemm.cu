@@ -107,7 +107,7 @@ struct TcCfg {
 struct TcArgs {
   const int32_t* seg;
   int E, N, K;
-  int row_tile;    // weight rows per set (<= 128, a multiple of 16): tc_row_tile
+  int row_tile;    // weight rows per set (96, 112 or 128): tc_row_tile
   int ntiles;      // row tiles per expert (N / row_tile for gate+up, N / 256 for down)
   int tok_tile;    // upper bound on tokens per tile (multiple of 16, <= 192)
   int ksplit;      // k partitions per tile (down only); partial kc goes to out + kc*P*N
@@ -839,20 +839,24 @@ double tc_expected_token_tiles(int pairs, int experts, int tok_tile) {
 }
 
 // Rows of each weight set per gate/up tile.  The narrow token tiles stream their
-// weights, so a tile's time is its rows' (+ about 8 rows' worth at the boundary)
-// and what counts is the last wave of SMs: of the heights that divide the matrix
-// take the one with the least rows over all waves.  Eight experts of 14336 rows: 896
-// tiles of 128 rows are 7 waves for 6.05 waves of work, 1024 tiles of 112 rows 6.92.
+// weights, so a tile's time is its rows' bytes (+ about 8 rows' worth at the boundary)
+// but no less than the dequant warps take for their 128 lanes, ~620 clocks per 64-k
+// stage = the bytes of 104 Q8_0 rows, and more than any 4-bit tile's bytes.  What
+// counts is the sum over the waves of SMs: eight experts of 14336 rows are 896 tiles of
+// 128 rows = 7 waves for 6.05 waves of work, or 1024 tiles of 112 rows = 6.92 waves of
+// shorter tiles (gate/up at 128 tokens 195 -> 167 us).  Tiles of 64 rows lose even where
+// they fill the waves: Q4_K, 2 tokens, ffn 16384, 7 waves of 64 rows 181 us, the
+// streaming kernel 115.
 // The 192-token variant is bound by its MMAs, which always work on 128 rows.
-int tc_row_tile(int rows, double token_tiles, int tok_tile) {
-  if (tok_tile > 128) return TC_ROWS;
+int tc_row_tile(int rows, double token_tiles, int tok_tile, bool q4) {
+  if (tok_tile > 128 || q4) return TC_ROWS;
   const int sms = sm_count();
   int best = TC_ROWS;
   double best_cost = 0.0;
-  for (int r = TC_ROWS; r >= 64; r -= 16) {
+  for (int r = TC_ROWS; r >= 96; r -= 16) {
     if (rows % r != 0) continue;
     const double waves = ceil(token_tiles * (rows / r) / sms);
-    const double cost = waves * (r + 8);
+    const double cost = waves * ((r > 104 ? r : 104) + 8);
     if (r == TC_ROWS || cost < 0.98 * best_cost) { best_cost = cost; best = r; }
   }
   return best;
@@ -916,7 +920,8 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
   if (pairs == 0) return B200MOE_OK;
   TcArgs a{};
   a.tok_tile = tc_pick_tok_tile(tok_tile, pairs, gate->experts);
-  a.row_tile = tc_row_tile(gate->rows, tc_expected_token_tiles(pairs, gate->experts, a.tok_tile), a.tok_tile);
+  a.row_tile = tc_row_tile(gate->rows, tc_expected_token_tiles(pairs, gate->experts, a.tok_tile), a.tok_tile,
+                           gate->layout == B200MOE_LAYOUT_Q4_K);
   CUtensorMap maps[12] = {};
   if (int rc = tc_weight_map(gate, &maps[0], &maps[2], a.row_tile)) return rc;
   if (int rc = tc_weight_map(up, &maps[1], &maps[3], a.row_tile)) return rc;

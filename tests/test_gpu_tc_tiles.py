@@ -11,7 +11,7 @@ from helpers import b200_block, device_input, oracle_params
 pytestmark = pytest.mark.gpu
 
 
-# ffn 1792 = 16 x 112 = 14 x 128, 768 = 12 x 64 = 8 x 96 = 6 x 128, 1280 = 10 x 128 = 20 x 64
+# ffn 1792 = 16 x 112 = 14 x 128, 768 = 8 x 96 = 6 x 128, 1280 = 10 x 128
 @pytest.mark.parametrize("kind", [syn.Q8_0, syn.Q4_K])
 @pytest.mark.parametrize("ffn,activation", [(1792, "silu"), (768, "gelu"), (1280, "silu")])
 @pytest.mark.parametrize("tokens", [1, 17, 129, 400])
