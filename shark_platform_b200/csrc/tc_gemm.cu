@@ -16,10 +16,10 @@
 //
 // Three independent shared-memory rings, because their slots live for very
 // different times:
-//   weights  2-5 slots x (2 sets x 128 rows x 128 k) int8, 128-byte swizzle;
+//   weights  2, 4 or 5 slots x (2 sets x 128 rows x 128 k) int8, 128-byte swizzle;
 //            a slot is free again as soon as the dequant warps have read it
-//   tokens   3 slots x (192 rows x 128 k) fp16; a slot is held until the MMAs
-//            that read it have completed
+//   tokens   2 or 3 slots x (64, 128 or 192 rows x 128 k) fp16; a slot is held until
+//            the MMAs that read it have completed
 //   scales   2 slots x (2 sets x 128 rows x 8) fp16 = 256 k
 //
 // Warp roles (608 threads, one CTA per SM, persistent over tiles):
@@ -87,11 +87,18 @@ struct TcCfg {
   // weight on both sides
   static constexpr int HK = NMAX <= 128 ? 2 : 1;
   static constexpr int HSLOTS = ASLOTS / HK;            // 3, 2, 2
-  static constexpr int WSLOTS = NMAX == 192 ? 2 : NMAX == 128 ? 3 : 5;
+  static constexpr int WSLOTS = NMAX == 192 ? 2 : NMAX == 128 ? 4 : 5;
+  // With HK = 2 a group waits on every second weight fill only.  An even ring keeps each
+  // slot with one group.  In an odd one the slots change groups, and a wait by parity
+  // also passes when the other group's fill of the slot, WSLOTS fills ago, has not landed
+  // yet.  What then vouches for that fill is the group's last hand-over, two fills ago: it
+  // needed the MMAs of the hand-over HSLOTS before it.  (Three slots with two hand-over
+  // slots broke this rule: stale weights, arrivals on a used-up phase.)
+  static_assert(HK == 1 || WSLOTS % 2 == 0 || HSLOTS + 2 <= WSLOTS, "a group could pass a slot that is still being filled");
   // a token slot holds two 64-k stages (two swizzled sub-tiles of NMAX rows x 128 B):
   // one wait and one release per 128 k on the issuing lanes, whose instruction
   // stream is the kernel's critical path
-  static constexpr int XSLOTS = 3;
+  static constexpr int XSLOTS = NMAX == 128 ? 2 : 3;
   static constexpr int XSUB = NMAX * TC_KT * 2;
   static constexpr int XSLOT = 2 * XSUB;
   static constexpr int OFF_X = WSLOTS * TC_WSLOT;
