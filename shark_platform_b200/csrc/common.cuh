@@ -161,7 +161,22 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
-// The same wait for a whole warp (all 32 lanes call it, converged).  Every lane
+// Wait, on the way out of a kernel, for a copy or an MMA that has been issued: it lands
+// whether or not the CTA has given up, so the abort flag is not looked at.  A CTA that left
+// before would hand its shared or tensor memory to the next one with writes still to come.
+// What is in flight lands within microseconds; the limit of ~2^26 clock ticks is for the
+// case that it never does.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, int32_t* status) {
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (clock64() - t0 > (1ll << 26)) {
+      atomicOr(status, DEV_ERR_WAIT_TIMEOUT);
+      return;
+    }
+  }
+}
+
+// mbar_wait for a whole warp (all 32 lanes call it, converged).  Every lane
 // runs its own bounded wait, so all of them come back; the vote then makes the
 // outcome uniform: when the abort flag is raised at the moment a phase completes,
 // one lane may see the phase and another the flag, and a warp that split on that

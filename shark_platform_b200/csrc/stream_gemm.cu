@@ -271,7 +271,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_const
       const uint32_t issued = n;
       const uint32_t first = issued > (uint32_t)STAGES ? issued - STAGES : 0;
       for (uint32_t i = first; i < issued; ++i)
-        mbar_wait(full_bar(i % STAGES), (i / STAGES) & 1u, abort_flag, args.status);
+        mbar_drain(full_bar(i % STAGES), (i / STAGES) & 1u, args.status);
     }
     return;
   }

@@ -47,7 +47,8 @@
 // columns each), two A staging slots of 2 x 32 columns at 384..511.
 //
 // All mbarrier waits are bounded; on expiry the CTA raises its abort flag, every
-// role falls out of its loops, the CTA frees its tensor memory and returns.
+// role falls out of its loops, its copies and MMAs in flight are waited for (bounded,
+// mbar_drain), the CTA frees its tensor memory and returns.
 #include <math.h>
 
 #include "common.cuh"
@@ -108,7 +109,7 @@ struct TcCfg {
   static constexpr uint32_t COL_ACC0 = 0, COL_ACC1 = NMAX, COL_A = 2 * NMAX;
   static_assert(XSLOT % 1024 == 0 && TC_WSLOT % 1024 == 0, "slot alignment for the swizzle");
   static_assert(SMEM <= 232448, "shared memory budget");
-  static_assert(2 * (WSLOTS + XSLOTS + TC_SSLOTS + 2 * HSLOTS) + 2 <= 64, "barrier area");
+  static_assert(2 * (WSLOTS + XSLOTS + TC_SSLOTS + 2 * HSLOTS) + 4 <= 64, "barrier area");
 };
 
 struct TcArgs {
@@ -346,6 +347,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const uint32_t sfull = take(TC_SSLOTS), sempty = take(TC_SSLOTS);
   const uint32_t a_ready = take(2 * HSLOTS), a_free = take(2 * HSLOTS);  // [slot][row set]
   const uint32_t acc_full_bar = take(1), acc_empty_bar = take(1);
+  const uint32_t mma_done = take(2);  // [row set]
 
   // the shuffle tells the compiler that the warp index is warp-uniform
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -369,6 +371,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     }
     mbar_init(acc_full_bar, 2);  // both issuers commit
     mbar_init(acc_empty_bar, TC_DQ_WARPS);  // one arrival per dequant warp
+    mbar_init(mma_done, 1);
+    mbar_init(mma_done + 8u, 1);
     fence_mbar_init();
   }
   if (warp == TC_WARP_MMA) {
@@ -425,6 +429,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // ------------------------------------------- TMA producer: weights + scales
     if (lane == 0) {
       uint32_t n = 0;  // global stage counter; weight slots advance every 2, scale slots every 4
+      uint32_t gn = 0;  // scale slots filled
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         int e, nt, row0, rows, ncols;
@@ -443,10 +448,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         for (int st = 0; st < stages_per_tile; st += 2, n += 2) {
           const int k0 = kbase + st * TC_KT;
           if (st % TC_SGROUP == 0) {
-            const uint32_t g = n / TC_SGROUP;
-            const int ss = g % TC_SSLOTS;
-            if (!mbar_wait(sempty + 8u * ss, ((g / TC_SSLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
+            const int ss = gn % TC_SSLOTS;
+            if (!mbar_wait(sempty + 8u * ss, ((gn / TC_SSLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
             fence_proxy_async_smem();
+            ++gn;
             const uint32_t sdst = scale_base + ss * TC_SSLOT;
             const uint32_t sb = sfull + 8u * ss;
             mbar_expect_tx(sb, 2 * SSET_BYTES);
@@ -476,10 +481,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // do not leave while copies may still land in this CTA's shared memory
       const uint32_t wn = n >> 1;
       for (uint32_t i = wn > (uint32_t)TC_WSLOTS ? wn - TC_WSLOTS : 0; i < wn; ++i)
-        mbar_wait(wfull + 8u * (i % TC_WSLOTS), (i / TC_WSLOTS) & 1u, abort_flag, args.status);
-      const uint32_t gn = n / TC_SGROUP;
+        mbar_drain(wfull + 8u * (i % TC_WSLOTS), (i / TC_WSLOTS) & 1u, args.status);
       for (uint32_t g = gn > (uint32_t)TC_SSLOTS ? gn - TC_SSLOTS : 0; g < gn; ++g)
-        mbar_wait(sfull + 8u * (g % TC_SSLOTS), (g / TC_SSLOTS) & 1u, abort_flag, args.status);
+        mbar_drain(sfull + 8u * (g % TC_SSLOTS), (g / TC_SSLOTS) & 1u, args.status);
     }
   } else if (warp == TC_WARP_XPROD) {
     // -------------------------------------------------- TMA producer: token tiles
@@ -506,7 +510,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         }
       }
       for (uint32_t i = n > (uint32_t)TC_XSLOTS ? n - TC_XSLOTS : 0; i < n; ++i)
-        mbar_wait(xfull + 8u * (i % TC_XSLOTS), (i / TC_XSLOTS) & 1u, abort_flag, args.status);
+        mbar_drain(xfull + 8u * (i % TC_XSLOTS), (i / TC_XSLOTS) & 1u, args.status);
     }
   } else if (warp == TC_WARP_MMA || warp == TC_WARP_MMA1) {
     // ------------------------------------------ MMA issuers, one per row set
@@ -551,6 +555,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       if (ok && elect_one()) tc_commit(acc_full_bar);
       __syncwarp();
     }
+    // after a wait that ran out nobody else waits for the last MMAs
+    if (elect_one()) tc_commit(mma_done + 8u * mset);
+    __syncwarp();
+    mbar_drain(mma_done + 8u * mset, 0, args.status);
   } else {
     // ------------------------------------- dequantise (both sets) + epilogue
     const int grp = warp >> 3;              // stage parity this warp works on

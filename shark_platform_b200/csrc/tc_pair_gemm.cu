@@ -178,10 +178,9 @@ __device__ __forceinline__ void tp_fence_before() {
 __device__ __forceinline__ void tp_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// arrives on the barrier at this shared-memory offset in both CTAs once all
-// MMAs issued so far have completed
-__device__ __forceinline__ void tp_commit_both(uint32_t bar) {
-  const uint16_t mask = 3;
+// arrives on the barrier at this shared-memory offset in the CTAs of the mask (both)
+// once all MMAs issued so far have completed
+__device__ __forceinline__ void tp_commit_both(uint32_t bar, uint16_t mask = 3) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       ::"r"(bar), "h"(mask)
@@ -262,7 +261,7 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
   const uint32_t xfull = take(TP_XSLOTS), xempty = take(TP_XSLOTS);
   const uint32_t sfull = take(TP_SSLOTS), sempty = take(TP_SSLOTS);
   const uint32_t a_ready = take(2), a_free = take(2);
-  const uint32_t acc_full_bar = take(1), acc_empty_bar = take(1);
+  const uint32_t acc_full_bar = take(1), acc_empty_bar = take(1), mma_done = take(1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();       // 0 = leader
@@ -288,6 +287,7 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       mbar_init(a_free + 8u * s, 1);
     }
     mbar_init(acc_full_bar, 1);
+    mbar_init(mma_done, 1);
     mbar_init(acc_empty_bar, 2 * TP_DQ_WARPS);  // leader only: one arrival per dequant warp of both CTAs
     fence_mbar_init();
     int run = 0;
@@ -344,7 +344,7 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
   if (warp == TP_WARP_WPROD) {
     // ------------------------------------------- TMA producer: weights + scales (per CTA)
     if (lane == 0) {
-      uint32_t n = 0;
+      uint32_t n = 0, gn = 0;  // stages, scale slots filled
       bool ok = true;
       for (int tile = pair; tile < total_tiles && ok; tile += npairs) {
         int e, nt, row0, rows, ncols;
@@ -356,10 +356,10 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         for (int st = 0; st < stages_per_tile; st += 2, n += 2) {
           const int k0 = kbase + st * TP_KT;
           if (st % TP_SGROUP == 0) {
-            const uint32_t g = n / TP_SGROUP;
-            const int ss = g % TP_SSLOTS;
-            if (!mbar_wait(sempty + 8u * ss, ((g / TP_SSLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
+            const int ss = gn % TP_SSLOTS;
+            if (!mbar_wait(sempty + 8u * ss, ((gn / TP_SSLOTS) & 1u) ^ 1u, abort_flag, args.status)) { ok = false; break; }
             fence_proxy_async_smem();
+            ++gn;
             const uint32_t sdst = scale_base + ss * TP_SSLOT;
             const uint32_t sb = sfull + 8u * ss;
             mbar_expect_tx(sb, 2 * SSET_BYTES);
@@ -390,10 +390,9 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       }
       const uint32_t wn = n >> 1;
       for (uint32_t i = wn > (uint32_t)TP_WSLOTS ? wn - TP_WSLOTS : 0; i < wn; ++i)
-        mbar_wait(wfull + 8u * (i % TP_WSLOTS), (i / TP_WSLOTS) & 1u, abort_flag, args.status);
-      const uint32_t gn = n / TP_SGROUP;
+        mbar_drain(wfull + 8u * (i % TP_WSLOTS), (i / TP_WSLOTS) & 1u, args.status);
       for (uint32_t g = gn > (uint32_t)TP_SSLOTS ? gn - TP_SSLOTS : 0; g < gn; ++g)
-        mbar_wait(sfull + 8u * (g % TP_SSLOTS), (g / TP_SSLOTS) & 1u, abort_flag, args.status);
+        mbar_drain(sfull + 8u * (g % TP_SSLOTS), (g / TP_SSLOTS) & 1u, args.status);
     }
   } else if (warp == TP_WARP_XPROD) {
     // ------------------------ TMA producer: this CTA's half of the token tile
@@ -419,9 +418,15 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                            my_row0, xfull_leader + 8u * xs);
         }
       }
-      if (leader)
+      if (leader) {
         for (uint32_t i = n > (uint32_t)TP_XSLOTS ? n - TP_XSLOTS : 0; i < n; ++i)
-          mbar_wait(xfull + 8u * (i % TP_XSLOTS), (i / TP_XSLOTS) & 1u, abort_flag, args.status);
+          mbar_drain(xfull + 8u * (i % TP_XSLOTS), (i / TP_XSLOTS) & 1u, args.status);
+      } else if (!ok) {
+        // this CTA's copies complete on the leader's barriers, and a leader that gave up
+        // earlier does not wait for the newest: about a millisecond for them to land
+        const long long t0 = clock64();
+        while (clock64() - t0 < (1ll << 21)) {}
+      }
     }
   } else if (warp == TP_WARP_MMA) {
     // ------------------------------------------- MMA issuer (leader CTA only)
@@ -458,6 +463,9 @@ tc_pair_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         }
         if (ok) tp_commit_both(acc_full_bar);
       }
+      // after a wait that ran out nobody else waits for the last MMAs
+      tp_commit_both(mma_done, 1);  // the leader's own
+      mbar_drain(mma_done, 0, args.status);
     }
   } else {
     // ------------------------------------- dequantise (both sets) + epilogue, per CTA

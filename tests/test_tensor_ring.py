@@ -216,3 +216,16 @@ def test_rule_of_the_static_assert(WSLOTS, HSLOTS):
             bad += 1
     safe = WSLOTS % 2 == 0 or HSLOTS + 2 <= WSLOTS
     assert (bad == 0) == safe, bad
+
+
+@pytest.mark.parametrize("name", ["tc_gemm.cu", "tc_pair_gemm.cu", "stream_gemm.cu"])
+def test_no_kernel_leaves_with_copies_in_flight(name):
+    """After a wait that ran out, mbar_wait returns at once: a producer's last waits for its
+    own copies, and an issuer's for its MMAs, are mbar_drain, which ignores the abort flag."""
+    text = open(os.path.join(os.path.dirname(SOURCE), name)).read()
+    drains = re.findall(r"for \(uint32_t \w+ = [^;]+; \w+ < \w+; \+\+\w+\)\s*\n\s*(\w+)\(", text)
+    assert drains and set(drains) == {"mbar_drain"}
+    if name != "stream_gemm.cu":
+        assert re.search(r"commit\w*\(mma_done[^\n]*\n(\s*__syncwarp\(\);\n)?\s*mbar_drain\(mma_done", text)
+        # a scale slot is filled before the wait for its weights can run out: counted by itself
+        assert "++gn;" in text and not re.search(r"gn = n /", text)
