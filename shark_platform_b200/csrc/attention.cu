@@ -728,7 +728,7 @@ __global__ void __launch_bounds__(AD_THREADS) attn_decode_mma_kernel(const Decod
 
 // Merges the splits: out[b, head, d] = sum_s acc_s * exp(m_s - M) / sum_s l_s * exp(m_s - M).
 __global__ void __launch_bounds__(128)
-attn_decode_merge_kernel(const float* __restrict__ partial, int splits, int G, int hd, int heads, int kv_heads,
+attn_decode_merge_kernel(const float* partial, int splits, int G, int hd, int heads, int kv_heads,
                          void* __restrict__ out, int out_dtype) {
   grid_dep_wait();
   grid_dep_launch();

@@ -83,7 +83,10 @@ cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t s
 }
 
 // Waits until the kernels before this one in the stream have completed and their
-// writes are visible.  A no-op in a kernel launched the ordinary way.
+// writes are visible.  A no-op in a kernel launched the ordinary way.  What an earlier
+// kernel writes is not declared __restrict__: a const __restrict__ pointer promises that
+// nothing writes there while this kernel runs, and loads through it could move up past
+// this wait.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next kernel of the stream start once every block has said so (or ended).
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

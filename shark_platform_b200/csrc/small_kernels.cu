@@ -237,8 +237,7 @@ constexpr long long RP_MAX_COUNTS = 16384;
 template <typename T>
 __global__ void __launch_bounds__(RP_THREADS)
 route_permute_kernel(const T* __restrict__ h, int tokens, int d, int E, int k,
-                     const float* __restrict__ norm_w, const float* __restrict__ rstd,
-                     const int32_t* __restrict__ experts, const int32_t* __restrict__ hist,
+                     const float* __restrict__ norm_w, const float* rstd, const int32_t* experts, const int32_t* hist,
                      int32_t* __restrict__ counts, int32_t* __restrict__ seg, int32_t* __restrict__ perm,
                      int32_t* __restrict__ inv, int kperm, uint4* __restrict__ xs) {
   __shared__ int s_total[MAX_EXPERTS], s_before[MAX_EXPERTS], s_seg[MAX_EXPERTS + 1];
@@ -984,7 +983,7 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, const fl
 // gate-weighted sum over the token's slots for four columns; per element the
 // same operations in the same order as a scalar loop over slots and partials
 template <typename TD>
-__device__ __forceinline__ void combine4(const TD* __restrict__ dpart, int ksplit, size_t part_stride,
+__device__ __forceinline__ void combine4(const TD* dpart, int ksplit, size_t part_stride,
                                          const int (&pos)[MAX_TOPK], const float (&gate)[MAX_TOPK],
                                          int k, int d, int j, float (&acc)[4]) {
 #pragma unroll
@@ -1007,8 +1006,7 @@ __device__ __forceinline__ void combine4(const TD* __restrict__ dpart, int kspli
 
 template <typename TD, typename TH, typename TY>
 __global__ void __launch_bounds__(COMBINE_THREADS)
-combine_kernel(const TD* __restrict__ dpart, int ksplit, size_t part_stride,
-               const int32_t* __restrict__ inv, const float* __restrict__ gates,
+combine_kernel(const TD* dpart, int ksplit, size_t part_stride, const int32_t* inv, const float* gates,
                const TH* __restrict__ h, int d, int k, const float* __restrict__ out_norm_w,
                float eps, int add_residual, TY* __restrict__ y) {
   extern __shared__ float s_row[];

@@ -212,3 +212,22 @@ def test_debug_flags_parse_like_the_reference_switch():
     assert not dbg.DebugFlags.parse("").any
     with pytest.raises(ValueError):
         dbg.DebugFlags.parse("no_such_flag")
+
+
+def test_dependent_kernels_promise_nothing_about_earlier_kernels_results():
+    """A kernel with grid_dep_wait() runs while the one before it still writes: `const
+    __restrict__` is for weights and for the caller's input only."""
+    import glob
+    import re
+
+    csrc = os.path.join(os.path.dirname(__file__), "..", "shark_platform_b200", "csrc")
+    seen = 0
+    for path in glob.glob(os.path.join(csrc, "*.cu")):
+        text = open(path).read()
+        for m in re.finditer(r"__global__ void[^{;]*?\((?P<args>[^{]*)\)\s*\{(?P<body>.*?)\n\}", text, re.S):
+            if "grid_dep_wait();" not in m["body"]:
+                continue
+            seen += 1
+            inputs = set(re.findall(r"const \w+\* ?__restrict__ (\w+)", m["args"]))
+            assert inputs <= {"norm_w", "out_norm_w", "h"}, (os.path.basename(path), inputs)
+    assert seen >= 8
