@@ -318,8 +318,11 @@ int b200moe_ep_layer_forward(const b200moe_layer_t* layer, const b200moe_ep_t* e
                              int32_t ret_rows, int32_t max_segment, int32_t ksplit, int32_t epoch,
                              void* workspace, size_t workspace_bytes, void* stream);
 
-/* Bytes of workspace b200moe_layer_forward needs for up to `tokens` tokens. */
+/* Bytes of workspace b200moe_layer_forward needs for up to `tokens` tokens: the most of
+ * all counts from 1 to `tokens` (a smaller call can need more than a larger one).
+ * b200moe_call_workspace_bytes: for a call of exactly `tokens` tokens. */
 size_t b200moe_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens);
+size_t b200moe_call_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens);
 
 /* Whole MoeBlock.forward (layers/mixture_of_experts_block.py:64-90) on one
  * device: router -> route plan -> permute -> gate/up -> down -> combine.

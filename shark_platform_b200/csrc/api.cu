@@ -168,12 +168,10 @@ struct Workspace {
   size_t bytes;
 };
 
-Workspace carve(const b200moe_layer_t* L, int tokens, void* base) {
+Workspace carve_rows(const b200moe_layer_t* L, int tokens, size_t part_rows, void* base) {
   const size_t T = tokens > 0 ? tokens : 1;
   const size_t P = T * L->top_k;
   const size_t d = L->hidden, F = L->ffn;
-  int ks = stream_down_ksplit(&L->down, static_cast<int>(P));
-  if (tc_supported(&L->down, true)) ks = max(ks, tc_down_ksplit(&L->down, static_cast<int>(P)));
   uint8_t* p = static_cast<uint8_t*>(base);
   size_t off = 0;
   auto take = [&](size_t n) {
@@ -191,9 +189,17 @@ Workspace carve(const b200moe_layer_t* L, int tokens, void* base) {
   w.inv = static_cast<int32_t*>(take(P * 4));
   w.xs = static_cast<__half*>(take(P * d * 2));
   w.a = static_cast<__half*>(take(P * F * 2));
-  w.dpart = static_cast<float*>(take(static_cast<size_t>(ks) * P * d * 4));
+  w.dpart = static_cast<float*>(take(part_rows * d * 4));
   w.bytes = off;
   return w;
+}
+
+// For a call of exactly `tokens` tokens, in either regime.
+Workspace carve(const b200moe_layer_t* L, int tokens, void* base) {
+  const size_t P = static_cast<size_t>(tokens > 0 ? tokens : 1) * L->top_k;
+  int ks = stream_down_ksplit(&L->down, static_cast<int>(P));
+  if (tc_supported(&L->down, true)) ks = max(ks, tc_down_ksplit(&L->down, static_cast<int>(P)));
+  return carve_rows(L, tokens, ks * P, base);
 }
 
 int check_layer(const b200moe_layer_t* L) {
@@ -428,6 +434,20 @@ int b200moe_combine(const void* d_partials, int d_dtype, int32_t ksplit, int32_t
 }
 
 size_t b200moe_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens) {
+  if (layer == nullptr || tokens < 0) return 0;
+  // A smaller call can need more (its k split is larger): the most of all counts, from
+  // the top down to where even the largest number of partial rows would not reach it.
+  size_t most = carve(layer, tokens, nullptr).bytes;
+  const size_t extra = max(stream_down_extra_rows(), tc_supported(&layer->down, true) ? tc_down_extra_rows(&layer->down) : 0);
+  for (int t = tokens - 1; t > 0; --t) {
+    const size_t P = static_cast<size_t>(t) * layer->top_k;
+    if (carve_rows(layer, t, P + min(7 * P, extra), nullptr).bytes <= most) break;
+    most = max(most, carve(layer, t, nullptr).bytes);
+  }
+  return most;
+}
+
+size_t b200moe_call_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens) {
   if (layer == nullptr || tokens < 0) return 0;
   return carve(layer, tokens, nullptr).bytes;
 }

@@ -41,6 +41,7 @@ int launch_gguf_q4k(const uint8_t* raw, long long blocks, void* d, void* dmin, u
 
 // decode regime (stream_gemm.cu)
 int stream_down_ksplit(const b200moe_weight_t* down, int pairs);
+size_t stream_down_extra_rows();  // bound of (k split - 1) * pairs over all pair counts
 int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max_segment,
                           const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
                           int out_kperm, int prefetch, void* a_out, cudaStream_t st);
@@ -58,6 +59,7 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
                       const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,
                       int out_kperm, int prefetch, void* a_out, cudaStream_t st);
 int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs);
+size_t tc_down_extra_rows(const b200moe_weight_t* down);  // as stream_down_extra_rows
 int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile,
                    const b200moe_weight_t* down, int ksplit, int prefetch, float* d_out, cudaStream_t st);
 

@@ -608,13 +608,16 @@ int check_weight(const b200moe_weight_t* w, const char* name) {
 
 }  // namespace
 
+constexpr int ST_SPLIT_MAX_PAIRS = 1024;
 int stream_down_ksplit(const b200moe_weight_t* down, int pairs) {
   const int stages = down->cols / KT;
-  if (pairs > 1024) return 1;
+  if (pairs > ST_SPLIT_MAX_PAIRS) return 1;
   if (stages % 4 == 0 && stages >= 8) return 4;
   if (stages % 2 == 0 && stages >= 4) return 2;
   return 1;
 }
+
+size_t stream_down_extra_rows() { return 3 * ST_SPLIT_MAX_PAIRS; }
 
 int launch_stream_gate_up(const void* xs, const int32_t* seg, int pairs, int max_segment,
                           const b200moe_weight_t* gate, const b200moe_weight_t* up, int act,

@@ -848,7 +848,9 @@ double tc_expected_token_tiles(int pairs, int experts, int tok_tile) {
   const double mean = static_cast<double>(pairs) / (experts > 0 ? experts : 1);
   const double sd = mean > 1.0 ? sqrt(mean) : 1.0;
   double tiles = 1.0;
-  for (int b = tok_tile; b < mean + 4.0 * sd; b += tok_tile)
+  int b = tok_tile;
+  for (; b < mean - 6.0 * sd; b += tok_tile) tiles += 1.0;  // passed for certain
+  for (; b < mean + 4.0 * sd; b += tok_tile)
     tiles += 0.5 * erfc((b + 0.5 - mean) / (1.4142135623730951 * sd));
   return tiles * (pairs < experts ? pairs : experts);
 }
@@ -957,6 +959,9 @@ int launch_tc_gate_up(const void* xs, const int32_t* seg, int pairs, int tok_til
   return tc_launch<B200MOE_LAYOUT_Q8_0, 2>(maps, a, st);
 }
 
+// Writing and reading back one row of partial sums at the copy bandwidth, in 64-k stages.
+static double tc_part_cost(int rows) { return rows * 8.0 / 6.5e6 / 0.4; }
+
 int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs) {
   // The long reduction is split into up to eight partitions when that fills the
   // waves of SMs better.  Cost in 64-k stages (about 0.4 us each): waves of items,
@@ -968,7 +973,7 @@ int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs) {
   const int sms = sm_count();
   const int tok = tc_pick_tok_tile(TC_NTOK, est_pairs, down->experts);
   const double tiles = tc_expected_token_tiles(est_pairs, down->experts, tok) * (down->rows / (2 * TC_ROWS));
-  const double part = static_cast<double>(est_pairs) * down->rows * 8.0 / 6.5e6 / 0.4;
+  const double part = static_cast<double>(est_pairs) * tc_part_cost(down->rows);
   int best = 1;
   double best_cost = 0.0;
   for (int ks = 1; ks <= 8; ks *= 2) {
@@ -977,6 +982,12 @@ int tc_down_ksplit(const b200moe_weight_t* down, int est_pairs) {
     if (ks == 1 || cost < 0.98 * best_cost) { best_cost = cost; best = ks; }
   }
   return best;
+}
+
+// A split is taken only where its partial sums cost less than the last wave can save:
+// ceil(x) < x + 1 in the cost above gives (ks - 1) * part < stages + 3.
+size_t tc_down_extra_rows(const b200moe_weight_t* down) {
+  return static_cast<size_t>((down->cols / TC_KT + 3) / tc_part_cost(down->rows)) + 1;
 }
 
 int launch_tc_down(const void* a_in, const int32_t* seg, int pairs, int tok_tile,
@@ -1039,7 +1050,7 @@ int tc_linear_ksplit(const b200moe_weight_t* const* w, int count, int rows) {
   const int sms = sm_count();
   const int tok = tc_linear_tok_tile(rows, row_tiles);
   const double tiles = static_cast<double>((rows + tok - 1) / tok) * row_tiles;
-  const double part = static_cast<double>(rows) * out_rows * 8.0 / 6.5e6 / 0.4;
+  const double part = rows * tc_part_cost(static_cast<int>(out_rows));
   int best = 1;
   double best_cost = 0.0;
   for (int ks = 1; ks <= 8; ks *= 2) {

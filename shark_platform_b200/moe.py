@@ -278,12 +278,9 @@ class PreparedLayer:
         self._workspace_tokens = 0
 
     def workspace(self, tokens: int) -> torch.Tensor:
-        # the k split of the down projection depends on the token count: fewer tokens
-        # can need more bytes than the largest call so far
-        if self._workspace is None or tokens != self._workspace_tokens:
-            nbytes = C.lib.b200moe_workspace_bytes(ctypes.byref(self.desc), tokens)
-            if self._workspace is None or nbytes > self._workspace.numel():
-                self._workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+        if self._workspace is None or tokens > self._workspace_tokens:
+            nbytes = C.lib.b200moe_workspace_bytes(ctypes.byref(self.desc), tokens)  # covers smaller calls
+            self._workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
             self._workspace_tokens = tokens
         return self._workspace
 

@@ -231,3 +231,34 @@ def test_dependent_kernels_promise_nothing_about_earlier_kernels_results():
             inputs = set(re.findall(r"const \w+\* ?__restrict__ (\w+)", m["args"]))
             assert inputs <= {"norm_w", "out_norm_w", "h"}, (os.path.basename(path), inputs)
     assert seen >= 8
+
+
+@pytest.mark.parametrize("hidden,ffn,experts,top_k,layout", [
+    (4096, 14336, 8, 2, "LAYOUT_Q8_0"), (6144, 32768, 8, 2, "LAYOUT_Q8_0"), (4096, 14336, 1, 1, "LAYOUT_Q4_K"),
+    (2048, 4096, 8, 2, "LAYOUT_Q4_K"), (2048, 1024, 64, 8, "LAYOUT_Q8_0"), (1024, 512, 4, 2, "LAYOUT_F16")])
+def test_workspace_of_a_count_covers_every_smaller_call(hidden, ffn, experts, top_k, layout):
+    """b200moe_workspace_bytes(n) is what a caller reserves for up to n tokens, although the
+    k split, and with it the bytes per row, can be larger at a smaller count."""
+    import ctypes
+
+    from shark_platform_b200 import _cabi as C
+
+    layer = C.LayerDesc()
+    layer.hidden, layer.ffn, layer.experts, layer.top_k = hidden, ffn, experts, top_k
+    lay = getattr(C, layout)
+    layer.gate = layer.up = _desc(lay, experts, ffn, hidden)
+    layer.down = _desc(lay, experts, hidden, ffn)
+    ref, most = ctypes.byref(layer), 0
+    for n in range(1, 4200):
+        call = C.lib.b200moe_call_workspace_bytes(ref, n)
+        most = max(most, call)
+        if n < 1200 or n % 50 == 0:
+            assert C.lib.b200moe_workspace_bytes(ref, n) == most, n
+        # the call itself reserves what either kernel's split writes
+        for regime in (C.REGIME_STREAM, C.REGIME_TENSOR):
+            if regime == C.REGIME_TENSOR and layout == "LAYOUT_F16":
+                continue
+            ks = C.lib.b200moe_down_ksplit(ctypes.byref(layer.down), n * top_k, n, regime)
+            assert call >= n * top_k * (ks * hidden * 4 + hidden * 2 + ffn * 2)
+    p = C.lib.b200moe_pipeline_bytes(ref, C.DT_BF16, 1024, 2)
+    assert p >= 4 * 1024 * hidden * 2 + C.lib.b200moe_workspace_bytes(ref, 1024)
