@@ -318,6 +318,11 @@ int b200moe_ep_layer_forward(const b200moe_layer_t* layer, const b200moe_ep_t* e
                              int32_t ret_rows, int32_t max_segment, int32_t ksplit, int32_t epoch,
                              void* workspace, size_t workspace_bytes, void* stream);
 
+/* Which kernel the two products of the expert-parallel call take: how = {gate/up regime, its segment
+ * bound, down regime, its segment bound}.  The streaming kernel's bound may be lower than
+ * max_segment (smaller chunks).  Host arithmetic only. */
+int b200moe_ep_products(const b200moe_layer_t* layer, int regime, int32_t max_segment, int32_t* how);
+
 /* Bytes of workspace b200moe_layer_forward needs for up to `tokens` tokens: the most of
  * all counts from 1 to `tokens` (a smaller call can need more than a larger one).
  * b200moe_call_workspace_bytes: for a call of exactly `tokens` tokens. */

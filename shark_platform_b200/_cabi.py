@@ -129,6 +129,7 @@ _PROTOS = {
     "b200moe_ep_barrier": (c_int, [POINTER(EpDesc), c_int32, _P, _P]),
     "b200moe_ep_dispatch": (c_int, [POINTER(EpDesc), _P, _P, _P, _P, c_int32, c_int32, c_int32, c_int32, c_int32, _P]),
     "b200moe_ep_return": (c_int, [POINTER(EpDesc), _P, c_int32, c_int32, _P, c_int32, c_int32, _P]),
+    "b200moe_ep_products": (c_int, [_L, c_int, c_int32, POINTER(c_int32)]),
     "b200moe_ep_workspace_bytes": (c_size_t, [_L, c_int32, c_int32, c_int32]),
     "b200moe_ep_layer_forward": (c_int, [_L, POINTER(EpDesc), _P, _P, c_int, c_int32, c_int, c_int32, c_int32,
                                          c_int32, c_int32, c_int32, _P, c_size_t, _P]),

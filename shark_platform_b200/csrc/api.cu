@@ -587,6 +587,22 @@ EpWorkspace ep_carve(const b200moe_layer_t* L, int tokens, int cap_rows, int ksp
 }
 }  // namespace
 
+int b200moe_ep_products(const b200moe_layer_t* L, int regime, int32_t max_segment, int32_t* how) {
+  B200_REQUIRE(L && how, "ep_products: NULL argument");
+  // The kernel follows the true bound, as the k split and the workspace do.  Chunk-size
+  // hint for the streaming kernel: its launchers take chunks one size below the caller's
+  // bound when they see four or more experts; a rank that holds fewer of a layer with at
+  // least four gets the same here (a segment longer than the chunk costs a second pass,
+  // nothing else).
+  const bool hint = L->gate.experts < 4 && L->experts >= 4 && max_segment > 16 && max_segment <= 64;
+  const b200moe_weight_t* const w[2] = {&L->gate, &L->down};
+  for (int i = 0; i < 2; ++i) {
+    how[2 * i] = pick_regime(regime, w[i], max_segment, i == 1);
+    how[2 * i + 1] = hint && how[2 * i] == B200MOE_REGIME_STREAM ? (max_segment + 1) / 2 : max_segment;
+  }
+  return B200MOE_OK;
+}
+
 size_t b200moe_ep_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens, int32_t cap_rows,
                                   int32_t ksplit) {
   if (layer == nullptr || tokens < 0 || cap_rows < 0 || ksplit < 1) return 0;
@@ -639,18 +655,13 @@ int b200moe_ep_layer_forward(const b200moe_layer_t* L, const b200moe_ep_t* ep, c
     return rc;
   if (int rc = b200moe_ep_barrier(ep, epoch + 2, nullptr, stream)) return rc;
   prof_mark(pc, 3, st);
-  // Chunk-size hint for the streaming kernel.  Its launchers take chunks one
-  // size below the caller's upper bound when they see four or more experts; a
-  // rank that holds fewer of a layer with at least four gets the same here (a
-  // segment longer than the chunk costs a second pass, nothing else).
-  int seg_hint = max_segment;
-  if (L->gate.experts < 4 && L->experts >= 4 && max_segment > 16 && max_segment <= 64)
-    seg_hint = (max_segment + 1) / 2;
-  if (int rc = b200moe_gate_up(recv_x, w.seg2, cap_rows, seg_hint, &L->gate, &L->up, L->activation,
-                               regime, kp_mid, w.a, stream))
+  int32_t how[4];
+  if (int rc = b200moe_ep_products(L, regime, max_segment, how)) return rc;
+  if (int rc = b200moe_gate_up(recv_x, w.seg2, cap_rows, how[1], &L->gate, &L->up, L->activation,
+                               how[0], kp_mid, w.a, stream))
     return rc;
   prof_mark(pc, 4, st);
-  if (int rc = b200moe_down(w.a, w.seg2, cap_rows, seg_hint, &L->down, regime, ksplit, w.dpart, stream))
+  if (int rc = b200moe_down(w.a, w.seg2, cap_rows, how[3], &L->down, how[2], ksplit, w.dpart, stream))
     return rc;
   prof_mark(pc, 5, st);
   if (int rc = b200moe_ep_return(ep, w.dpart, ksplit, cap_rows, w.seg2, L->hidden, ret_rows, stream))

@@ -262,3 +262,30 @@ def test_workspace_of_a_count_covers_every_smaller_call(hidden, ffn, experts, to
             assert call >= n * top_k * (ks * hidden * 4 + hidden * 2 + ffn * 2)
     p = C.lib.b200moe_pipeline_bytes(ref, C.DT_BF16, 1024, 2)
     assert p >= 4 * 1024 * hidden * 2 + C.lib.b200moe_workspace_bytes(ref, 1024)
+
+
+@pytest.mark.parametrize("layout", ["LAYOUT_Q8_0", "LAYOUT_Q4_K"])
+@pytest.mark.parametrize("local", [1, 2, 4, 8])
+def test_expert_parallel_chunk_hint_does_not_choose_the_kernel(local, layout):
+    """A rank with fewer than four experts asks the streaming kernel for smaller chunks; the
+    kernel itself follows the true segment bound, for which the k split was computed."""
+    import ctypes
+
+    from shark_platform_b200 import _cabi as C
+
+    lay = getattr(C, layout)
+    layer = C.LayerDesc()
+    layer.hidden, layer.ffn, layer.experts, layer.top_k = 4096, 14336, 8, 2
+    layer.gate = layer.up = _desc(lay, local, 14336, 4096)
+    layer.down = _desc(lay, local, 4096, 14336)
+    first = 24 if layout == "LAYOUT_Q4_K" and local >= 4 else 32
+    how = (ctypes.c_int32 * 4)()
+    for n in range(1, 200):
+        assert C.lib.b200moe_ep_products(ctypes.byref(layer), C.REGIME_AUTO, n, how) == 0
+        kernel = C.REGIME_TENSOR if n >= first else C.REGIME_STREAM
+        bound = (n + 1) // 2 if local < 4 and 16 < n < first else n
+        assert list(how) == [kernel, bound] * 2
+        ks = C.lib.b200moe_down_ksplit(ctypes.byref(layer.down), 2 * n, n, C.REGIME_AUTO)
+        assert ks == C.lib.b200moe_down_ksplit(ctypes.byref(layer.down), 2 * n, how[3], how[2])
+    assert C.lib.b200moe_ep_products(ctypes.byref(layer), C.REGIME_STREAM, 40, how) == 0
+    assert list(how) == [C.REGIME_STREAM, 20 if local < 4 else 40] * 2
