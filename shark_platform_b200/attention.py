@@ -117,7 +117,6 @@ class B200PagedAttentionBlock(torch.nn.Module):
         else:  # one fused projection
             self._wqkv = torch.cat([_moe._unbox(t) for t in (wq, wk, wv)], dim=0).contiguous()
         self._freqs = None
-        self._scratch = None
         self._desc = C.KvCacheDesc(cache.transformer_block_count, cache.block_seq_stride, head_count_kv, head_dim, 0)
 
     # ---------------------------------------------------------------- pieces
@@ -225,14 +224,14 @@ class B200PagedAttentionBlock(torch.nn.Module):
             direct = fused_out and _moe._layout_name(self._wo) == "BlockScaledLayout"
             out = torch.empty(bs, H * hd, dtype=torch.float16 if direct else h.dtype, device=dev)
             nbytes = C.lib.b200moe_attn_decode_scratch_bytes(ctypes.byref(self._desc), bs, H, max_len)
-            if self._scratch is None or self._scratch.numel() < nbytes or self._scratch.device != dev:
-                self._scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            # per call, as the layer's workspace: other streams and captured graphs have their own
+            scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
             with torch.cuda.device(dev):
                 C.check(C.lib.b200moe_attn_decode(
                     _p(q), _DT[q.dtype], _p(slab), _DT[slab.dtype], ctypes.byref(self._desc), self.block_index,
                     _p(page_ids), _p(seq_lens), bs, page_ids.shape[1], H, max_len, float(scale),
                     float(self.softcap) if self.softcap is not None else 0.0, _p(out), _DT[out.dtype],
-                    _p(self._scratch), self._scratch.numel(), _moe._stream()), "attn_decode")
+                    _p(scratch), nbytes, _moe._stream()), "attn_decode")
             attn = out.view(bs, 1, H * hd)
         else:
             qh = q.view(bs, sl, H, hd).transpose(1, 2)

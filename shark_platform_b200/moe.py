@@ -242,7 +242,7 @@ def grouped_matmul(xs: torch.Tensor, plan_seg: torch.Tensor, w: PreparedWeight, 
 
 # -------------------------------------------------------------- the layer
 class PreparedLayer:
-    """All device-side state of one MoE layer: descriptor, weights, workspace."""
+    """All device-side state of one MoE layer: descriptor and weights."""
 
     def __init__(self, theta, expert_count: int, expert_used_count: int, rms_epsilon: float,
                  activation: str):
@@ -274,15 +274,16 @@ class PreparedLayer:
             None if self.out_norm_w is None else self.out_norm_w.data_ptr(),
             self.gate.desc, self.up.desc, self.down.desc, 0,
         )
-        self._workspace: Optional[torch.Tensor] = None
-        self._workspace_tokens = 0
+        self._call_bytes: dict[int, int] = {}  # token count -> workspace bytes
 
     def workspace(self, tokens: int) -> torch.Tensor:
-        if self._workspace is None or tokens > self._workspace_tokens:
-            nbytes = C.lib.b200moe_workspace_bytes(ctypes.byref(self.desc), tokens)  # covers smaller calls
-            self._workspace = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-            self._workspace_tokens = tokens
-        return self._workspace
+        """Scratch of one call on the current stream.  Taken from the caching allocator per
+        call and not kept: calls on two streams would write the same buffers, and a captured
+        graph would go on using a buffer that a larger call has replaced."""
+        nbytes = self._call_bytes.get(tokens)
+        if nbytes is None:
+            nbytes = self._call_bytes[tokens] = C.lib.b200moe_call_workspace_bytes(ctypes.byref(self.desc), tokens)
+        return torch.empty(nbytes, dtype=torch.uint8, device=self.device)
 
     def forward(self, h: torch.Tensor, regime: int = C.REGIME_AUTO, want_routing: bool = False):
         _require_cuda(h, "h")
