@@ -753,20 +753,28 @@ attn_decode_merge_kernel(const float* partial, int splits, int G, int hd, int he
   }
 }
 
-int decode_splits(int bs, int kv_heads, int max_seq_len) {
-  // Two to three CTAs of 128 positions per step or more are resident per SM; ragged
-  // lengths want somewhat more CTAs than that, every split costs the merge a partial
-  // result.  us on one B200 at 2 / 3 / 4 / 6 CTAs per SM asked for: 32 sequences of up
-  // to 4096 positions 85 / 86 / 82 / 87, 32 x 1024 33 / 33 / 31 / 34, 8 x 2048
-  // 24 / 21 / 24 / 25, 1 x 8192 (37 / 56 / 64 / 64 splits) 25 / 28 / 33 / 33.
+// Position splits per (sequence, kv head) of the two decode kernels; every split costs the
+// merge a partial result.  All figures: one B200, kernel and merge, us.
+// 16-bit cache: the CTAs ask for three to four per SM (2 / 3 / 4 / 6 per SM, with a ring
+// shared by the block: 32 sequences of up to 4096 positions 85 / 86 / 82 / 87, 32 x 1024
+// 33 / 33 / 31 / 34, 8 x 2048 24 / 21 / 24 / 25), at most 32 of them (1 x 8192, 8 kv heads,
+// L2 flushed: 16 / 32 / 48 / 64 splits 24 / 26 / 30 / 42), up to 64 only where even those
+// leave SMs idle and each still has 512 positions (1 and 2 kv heads, 32 / 64 splits: 8192
+// positions 24 / 28, 32768 positions 36 / 34).
+// fp32 cache: scalar products, long steps; six CTAs per SM, up to 64 splits (1 kv head,
+// 32 / 64 splits: 8192 positions 69 / 46, 32768 positions 232 / 128; 8 sequences x 8 kv
+// heads of 32768: 7 / 16 splits 2967 / 2351).
+int decode_splits(int bs, int kv_heads, int max_seq_len, bool f32) {
   const int base = bs * kv_heads;
-  const int per_sm = base >= sm_count() ? 4 : 3;
-  int splits = (per_sm * sm_count() + base - 1) / base;
+  const int sms = sm_count();
+  const int per_sm = f32 ? 6 : base >= sms ? 4 : 3;
+  int cap = 64;
+  if (!f32) cap = base * 64 <= sms && max_seq_len / 512 > 32 ? (max_seq_len / 512 < 64 ? max_seq_len / 512 : 64) : 32;
+  int splits = (per_sm * sms + base - 1) / base;
   const int most = (max_seq_len + AD_THREADS - 1) / AD_THREADS;
   if (splits > most) splits = most;
-  if (splits < 1) splits = 1;
-  if (splits > 32) splits = 32;
-  return splits;
+  if (splits > cap) splits = cap;
+  return splits < 1 ? 1 : splits;
 }
 
 template <typename TC, int HD>
@@ -858,7 +866,10 @@ int b200moe_attn_rope_kv_write(void* q, const void* k, const void* v, void* k_ou
 size_t b200moe_attn_decode_scratch_bytes(const b200moe_kv_cache_t* cache, int32_t bs, int32_t heads,
                                          int32_t max_seq_len) {
   if (cache == nullptr || bs <= 0 || heads <= 0 || cache->kv_heads <= 0 || heads % cache->kv_heads != 0) return 0;
-  const int splits = decode_splits(bs, cache->kv_heads, max_seq_len);
+  // the cache's type is not known here: enough for either kernel
+  const int s16 = decode_splits(bs, cache->kv_heads, max_seq_len, false);
+  const int s32 = decode_splits(bs, cache->kv_heads, max_seq_len, true);
+  const int splits = s16 > s32 ? s16 : s32;
   return static_cast<size_t>(bs) * heads * splits * (cache->head_dim + 2) * sizeof(float);
 }
 
@@ -891,7 +902,7 @@ int b200moe_attn_decode(const void* q, int q_dtype, const void* slab, int cache_
   a.partial = static_cast<float*>(scratch);
   a.bs = bs; a.heads = heads; a.kv_heads = cache->kv_heads; a.hd = cache->head_dim; a.stride = cache->stride;
   a.blocks = cache->blocks; a.block_index = block_index; a.pages_per_seq = pages_per_seq;
-  a.page_count = cache->page_count; a.splits = decode_splits(bs, cache->kv_heads, max_seq_len);
+  a.page_count = cache->page_count; a.splits = decode_splits(bs, cache->kv_heads, max_seq_len, cache_dtype == B200MOE_DT_F32);
   a.scale = scale; a.softcap = softcap; a.status = status;
   const dim3 grid(a.splits, a.kv_heads, bs);
   const int hd = cache->head_dim;

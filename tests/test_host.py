@@ -289,3 +289,22 @@ def test_expert_parallel_chunk_hint_does_not_choose_the_kernel(local, layout):
         assert ks == C.lib.b200moe_down_ksplit(ctypes.byref(layer.down), 2 * n, how[3], how[2])
     assert C.lib.b200moe_ep_products(ctypes.byref(layer), C.REGIME_STREAM, 40, how) == 0
     assert list(how) == [C.REGIME_STREAM, 20 if local < 4 else 40] * 2
+
+
+def test_decode_attention_scratch_allows_64_splits_of_a_long_context():
+    """Few kv heads and a long context: 32 position splits would leave most SMs idle."""
+    import ctypes
+
+    from shark_platform_b200 import _cabi as C
+
+    def splits(bs, kv_heads, positions, hd=128, group=8):
+        desc = C.KvCacheDesc(2, 32, kv_heads, hd, 100)
+        n = C.lib.b200moe_attn_decode_scratch_bytes(ctypes.byref(desc), bs, kv_heads * group, positions)
+        per = bs * kv_heads * group * (hd + 2) * 4
+        assert n % per == 0
+        return n // per
+
+    assert splits(1, 1, 65536) == 64 and splits(1, 2, 32768) == 64
+    assert splits(1, 1, 1000) == 8     # no split shorter than 128 positions
+    assert splits(1, 1, 100) == 1
+    assert splits(64, 8, 4096) >= 1
