@@ -124,6 +124,7 @@ class AttnParams:
     softcap: Optional[float] = None
     attention_scale: Optional[float] = None
     out_norm_w: Optional[torch.Tensor] = None
+    bias: Optional[dict] = None  # "q", "k", "v", "o" -> bias of that projection (ops.linear adds it)
 
 
 def _rms_norm(x, w, eps):
@@ -142,9 +143,10 @@ def attention_block(h: torch.Tensor, p: AttnParams, slab: torch.Tensor, geo: Cac
     bs, sl, d = h.shape
     H, Hkv, hd = p.head_count, p.head_count_kv, p.head_dim
     x = _rms_norm(h, p.norm_w, p.eps)
-    xq = (x @ p.wq.to(x.dtype).mT).view(bs, sl, H, hd)
-    xk = (x @ p.wk.to(x.dtype).mT).view(bs, sl, Hkv, hd)
-    xv = (x @ p.wv.to(x.dtype).mT).view(bs, sl, Hkv, hd)
+    bias = lambda name: 0.0 if p.bias is None or name not in p.bias else p.bias[name]
+    xq = (x @ p.wq.to(x.dtype).mT + bias("q")).view(bs, sl, H, hd)
+    xk = (x @ p.wk.to(x.dtype).mT + bias("k")).view(bs, sl, Hkv, hd)
+    xv = (x @ p.wv.to(x.dtype).mT + bias("v")).view(bs, sl, Hkv, hd)
     if start_positions is None:
         pos = torch.arange(sl).unsqueeze(0).expand(bs, sl)
     else:
@@ -171,7 +173,7 @@ def attention_block(h: torch.Tensor, p: AttnParams, slab: torch.Tensor, geo: Cac
         w = w + attention_mask
     w = torch.softmax(w.to(torch.float32), dim=-1).to(q.dtype)
     out = torch.matmul(w, values).transpose(1, 2).flatten(2, 3)
-    out = out @ p.wo.to(out.dtype).mT
+    out = out @ p.wo.to(out.dtype).mT + bias("o")
     if p.out_norm_w is not None:
         out = _rms_norm(out, p.out_norm_w, p.eps)
     return h + out

@@ -113,3 +113,31 @@ def test_rope_vector_path_equals_the_scalar_path(dtype, hd, heads, kv_heads, tok
                         x[..., 1::2] * ang.cos()[:, None] + x[..., 0::2] * ang.sin()[:, None]], -1).flatten(-2)
     # fp32 angles of up to 937 rad carry an absolute error of 937 * 2^-24
     assert orc.rel_l2(got[dtype][0].cpu().double(), want) < torch.finfo(dtype).eps
+
+
+# K of 256 and 768 leaves k unsplit: from 32 rows on the tensor kernel's drain rounds, adds
+# the residual and stores by itself (31 rows: the streaming kernel and the finish kernel)
+@pytest.mark.parametrize("k", [256, 768])
+@pytest.mark.parametrize("rows", [31, 32, 97, 385])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kinds", [(syn.Q8_0,), (syn.Q4_K,) * 3, (syn.Q8_0,) * 3])
+def test_unsplit_linears_write_finished_outputs(k, rows, dtype, kinds):
+    from shark_platform_b200 import moe
+
+    sizes = (512, 256, 256)
+    pairs = [_weight(kind, n, k, 90 + i) for i, (kind, n) in enumerate(zip(kinds, sizes))]
+    gen = torch.Generator().manual_seed(rows + k)
+    x = torch.randn(rows, k, generator=gen)
+    prep = [moe.prepare_linear(w) for w, _ in pairs]
+    for x_dtype in (torch.float32, torch.float16):
+        xs = x.to(x_dtype)
+        outs = moe.linear_rows(xs.cuda(), prep, out_dtype=dtype)
+        for out, (_, dense) in zip(outs, pairs):
+            assert out.dtype == dtype
+            assert orc.rel_l2(out.cpu().double(), xs.double() @ dense.mT) < TOL[dtype]
+        res = torch.randn(rows, sizes[0], generator=gen).to(dtype).cuda()
+        plus = moe.linear_rows(xs.cuda(), prep, residual=res, out_dtype=dtype)
+        assert torch.equal(plus[0], outs[0] + res)
+        for a, b in zip(plus[1:], outs[1:]):
+            assert torch.equal(a, b)
+    assert moe.device_status() == 0

@@ -90,3 +90,20 @@ def test_prefill_front_routes_as_the_oracle(experts, top_k, tokens, act_dtype):
     assert clear.float().mean() > 0.9
     assert torch.equal(ex.cpu().to(torch.int64)[clear], mid["experts"][clear])
     assert orc.rel_l2(y.float().cpu().reshape(tokens, -1)[clear], want.reshape(tokens, -1)[clear]) < 2e-2
+
+
+# one token to each side of where the tensor kernel takes over: 32, and 24 for 4-bit stacks
+# of four or more experts
+@pytest.mark.parametrize("kind,experts,first", [(syn.Q8_0, 8, 32), (syn.Q4_K, 8, 24), (syn.Q4_K, 2, 32)])
+@pytest.mark.parametrize("tokens", [23, 24, 31, 32])
+def test_change_over_between_the_kernels(kind, experts, first, tokens):
+    from shark_platform_b200 import moe
+
+    spec = syn.CaseSpec("change", tokens, 512, 1024, experts, 2, kind=kind, norm_weight="perturbed", seed=75)
+    case = syn.make_case(spec)
+    h = device_input(case)
+    got = b200_block(case)(h)
+    assert torch.equal(got, b200_block(case, regime="tensor" if tokens >= first else "stream")(h))
+    assert moe.device_status() == 0
+    want, _ = orc.moe_block(case.h, oracle_params(case), form="per_expert")
+    assert orc.rel_l2(got.float().cpu(), want) < 2e-2
