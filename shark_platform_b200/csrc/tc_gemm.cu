@@ -95,6 +95,10 @@ struct TcCfg {
   // yet.  What then vouches for that fill is the group's last hand-over, two fills ago: it
   // needed the MMAs of the hand-over HSLOTS before it.  (Three slots with two hand-over
   // slots broke this rule: stale weights, arrivals on a used-up phase.)
+  // What 128-token tiles could take instead: one-stage hand-overs with three weight and
+  // three token slots.  One B200, Q8_0, gate/up + down, us, 4 + 2 slots as here / that:
+  // 200 tokens 237 + 115 / 244 + 126, 320 tokens 267 + 135 / 261 + 131, 387 tokens
+  // 296 + 140 / 278 + 136; q, k and v of 41 to 96 rows 16.5 .. 21.2 / 17.9 .. 21.7.
   static_assert(HK == 1 || WSLOTS % 2 == 0 || HSLOTS + 2 <= WSLOTS, "a group could pass a slot that is still being filled");
   // a token slot holds two 64-k stages (two swizzled sub-tiles of NMAX rows x 128 B):
   // one wait and one release per 128 k on the issuing lanes, whose instruction
@@ -194,18 +198,8 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem descriptor]
-__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The four K=16 MMAs of a 64-k stage in one statement: A at a_tmem + 8 j columns,
-// B descriptors differing in the start-address field only (32 bytes = 2 units
+// D[tmem] (+)= A[tmem] * B[smem descriptor], the four K=16 MMAs of a 64-k stage in one
+// statement: A at a_tmem + 8 j columns, B descriptors differing in the start-address field only (32 bytes = 2 units
 // per K step; the upper descriptor word is constant).  The first one overwrites
 // the accumulator when `accumulate` is 0.
 __device__ __forceinline__ void tc_mma_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo,
@@ -281,8 +275,9 @@ __device__ __forceinline__ uint32_t make_idesc(int m, int n) {
 // of the earlier kernels may be read.  With PREFETCH_SEGMENTS the segment offsets are
 // those of a kernel that had completed before the one just ahead of us started; they
 // are read past L1 and, should they be stale all the same, only steer the prefetch to
-// other rows of the same matrix.  TC_PREFETCH stages: the ring's and a few more, about
-// what HBM delivers while the previous kernel drains.
+// other rows of the same matrix.  The first TC_PREFETCH_K columns of the tile's k part: what
+// the weight ring holds and a few slots more, about what HBM delivers while the previous
+// kernel drains.
 constexpr int TC_PREFETCH_K = 1536;
 template <int LAYOUT, int NMAT>
 __device__ __forceinline__ void tc_prefetch(const CUtensorMap& tm_w0, const CUtensorMap& tm_w1, const TcArgs& args) {
