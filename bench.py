@@ -409,12 +409,6 @@ def measure_layer(C, moe, syn, block, h, spec, args, peaks, sampler=None, cold=T
     return out
 
 
-def _layer_launches(fused, tokens, experts):
-    """Kernels of one single-GPU layer call: front (1 launch; 2 in prefill, 3 where the
-    router's expert counts outgrow the second kernel), gate/up, down, combine."""
-    return 4 if fused else 5 if -(-tokens // 4) * experts <= 16384 else 6
-
-
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -537,8 +531,7 @@ def main():
         case = syn.make_case(spec, tokens=tokens)
         block = syn.case_block(case, args.regime, dev)
         h = syn.case_input(case, dev).reshape(tokens, spec.hidden).contiguous()
-        fused = C.lib.b200moe_front_supported(tokens, ctypes.byref(block.layer.desc))
-        launches_per_step = _layer_launches(fused, tokens, block.layer.expert_count)
+        launches_per_step = C.lib.b200moe_layer_launches(ctypes.byref(block.layer.desc), tokens)
         m = measure_layer(C, moe, syn, block, h, spec, args, peaks, sampler)
         clocks = m["clocks"]
         if args.workload == "prefill4096" and not args.no_secondary:
@@ -577,8 +570,7 @@ def main():
         case0 = syn.make_case_on_device(dataclasses.replace(spec, tokens=tokens, seed=999), dev)
         h = syn.case_input(case0, dev).reshape(tokens, spec.hidden).contiguous()
         step = lambda: stack(h)
-        fused = C.lib.b200moe_front_supported(tokens, ctypes.byref(blocks[0].layer.desc))
-        launches_per_step = _layer_launches(fused, tokens, blocks[0].layer.expert_count) * layers
+        launches_per_step = C.lib.b200moe_layer_launches(ctypes.byref(blocks[0].layer.desc), tokens) * layers
         for _ in range(args.warmup):
             step()
         torch.cuda.synchronize()

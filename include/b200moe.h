@@ -336,6 +336,11 @@ int b200moe_layer_forward(const b200moe_layer_t* layer, const void* h, void* y, 
                           int32_t tokens, int regime, void* workspace, size_t workspace_bytes,
                           int32_t* experts_out, float* gates_out, void* stream);
 
+/* Kernels that call launches for `tokens` tokens: the front end (one kernel at decode
+ * counts, two at prefill counts, three where the router's expert counts outgrow the second
+ * of those), gate/up, down, combine. */
+int b200moe_layer_launches(const b200moe_layer_t* layer, int32_t tokens);
+
 /* Same call with host buffers: copies h to the device, runs the layer and
  * copies y back on `stream` (pinned host memory makes the copies asynchronous).
  * dev_io: device scratch of at least 2*T*d*sizeof(io_dtype) bytes. */

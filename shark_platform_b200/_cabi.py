@@ -135,6 +135,7 @@ _PROTOS = {
                                          c_int32, c_int32, c_int32, _P, c_size_t, _P]),
     "b200moe_workspace_bytes": (c_size_t, [_L, c_int32]),
     "b200moe_call_workspace_bytes": (c_size_t, [_L, c_int32]),
+    "b200moe_layer_launches": (c_int, [_L, c_int32]),
     "b200moe_layer_forward": (c_int, [_L, _P, _P, c_int, c_int32, c_int, _P, c_size_t, _P, _P, _P]),
     "b200moe_layer_forward_host": (c_int, [_L, _P, _P, c_int, c_int32, c_int, _P, _P, c_size_t, _P]),
     "b200moe_rms_norm": (c_int, [_P, c_int, _P, c_int64, c_int32, c_float, _P, c_int, _P]),

@@ -452,6 +452,11 @@ size_t b200moe_call_workspace_bytes(const b200moe_layer_t* layer, int32_t tokens
   return carve(layer, tokens, nullptr).bytes;
 }
 
+int b200moe_layer_launches(const b200moe_layer_t* L, int32_t tokens) {
+  if (L == nullptr || tokens <= 0) return 0;
+  return 3 + (front_fused_supported(tokens, L) ? 1 : front_prefill_supported(tokens, L) ? 2 : 3);
+}
+
 int b200moe_layer_forward(const b200moe_layer_t* L, const void* h, void* y, int io_dtype,
                           int32_t tokens, int regime, void* workspace, size_t workspace_bytes,
                           int32_t* experts_out, float* gates_out, void* stream) {

@@ -308,3 +308,14 @@ def test_decode_attention_scratch_allows_64_splits_of_a_long_context():
     assert splits(1, 1, 1000) == 8     # no split shorter than 128 positions
     assert splits(1, 1, 100) == 1
     assert splits(64, 8, 4096) >= 1
+
+
+def test_launches_of_a_layer_call():
+    import ctypes
+
+    from shark_platform_b200 import _cabi as C
+
+    layer = C.LayerDesc()
+    layer.hidden, layer.ffn, layer.experts, layer.top_k = 4096, 14336, 8, 2
+    n = lambda tokens: C.lib.b200moe_layer_launches(ctypes.byref(layer), tokens)
+    assert [n(t) for t in (0, 1, 128, 129, 8192, 8193)] == [0, 4, 4, 5, 5, 6]
