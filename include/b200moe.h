@@ -337,8 +337,8 @@ int b200moe_layer_forward(const b200moe_layer_t* layer, const void* h, void* y, 
                           int32_t* experts_out, float* gates_out, void* stream);
 
 /* Kernels that call launches for `tokens` tokens: the front end (one kernel at decode
- * counts, two at prefill counts, three where the router's expert counts outgrow the second
- * of those), gate/up, down, combine. */
+ * counts, two at prefill counts, three between the two and where the router's expert
+ * counts outgrow the second of those), gate/up, down, combine. */
 int b200moe_layer_launches(const b200moe_layer_t* layer, int32_t tokens);
 
 /* Same call with host buffers: copies h to the device, runs the layer and

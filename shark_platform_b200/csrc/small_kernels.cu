@@ -673,6 +673,9 @@ int clear_front_sync(cudaStream_t st) {
   return B200MOE_OK;
 }
 
+// One CTA per token (router_block_kernel) instead of four tokens per CTA.
+static bool router_per_token(int tokens, int hidden) { return tokens <= 512 && hidden <= 8 * RB_THREADS * RB_MAXV; }
+
 int launch_router(const void* h, int h_dtype, int tokens, const b200moe_layer_t* L, void* xn,
                   int32_t* experts, float* gates, cudaStream_t st) {
   B200_REQUIRE(L->hidden % 256 == 0, "router: hidden (%d) must be a multiple of 256", L->hidden);
@@ -683,7 +686,7 @@ int launch_router(const void* h, int h_dtype, int tokens, const b200moe_layer_t*
   if (tokens == 0) return B200MOE_OK;
   B200_REQUIRE(h_dtype == B200MOE_DT_F32 || h_dtype == B200MOE_DT_BF16,
                "router: activations must be fp32 or bf16");
-  if (tokens <= 512 && L->hidden <= 8 * RB_THREADS * RB_MAXV) {
+  if (router_per_token(tokens, L->hidden)) {
     if (h_dtype == B200MOE_DT_F32)
       router_block_kernel<float><<<tokens, RB_THREADS, 0, st>>>(
           static_cast<const float*>(h), L->hidden, L->experts, L->top_k, L->rms_epsilon,
@@ -713,8 +716,18 @@ int launch_router(const void* h, int h_dtype, int tokens, const b200moe_layer_t*
 }
 
 // Above the fused front's token count, while the count rows stay small enough to be
-// read whole by every CTA of the second kernel.
+// read whole by every CTA of the second kernel, and where router_tokens_kernel has CTAs
+// enough: a quarter of the tokens, each with four rows and all router weights to read, are
+// slower than one CTA per token until the SMs fill, the later the longer the rows and the
+// more experts there are.  Whole call with a small ffn, one B200, us, three kernels (router,
+// plan, permutation) / two: hidden 4096, 8 experts, 129 / 256 / 320 / 448 tokens 47.7 / 54.4,
+// 56.5 / 59.8, 61.7 / 62.0, 68.5 / 66.5; hidden 6144 256 / 512 tokens 73.7 / 83.7, 104.7 / 104.0;
+// hidden 2048, 64 experts, top 8, 129 / 256 / 320 tokens 80.7 / 106, 103.5 / 112, 121 / 115;
+// hidden 1024, 8 experts, 160 / 512 tokens 31.0 / 30.4, 46.4 / 40.5.
 bool front_prefill_supported(int tokens, const b200moe_layer_t* L) {
+  if (router_per_token(tokens, L->hidden) &&
+      tokens < static_cast<long long>(L->hidden) * (64 + L->experts) / 832)
+    return false;
   return tokens > FRONT_MAX_TOKENS && L->hidden % 256 == 0 && L->experts >= 1 && L->experts <= MAX_EXPERTS &&
          L->top_k >= 1 && L->top_k <= MAX_TOPK && L->top_k <= L->experts &&
          static_cast<long long>((tokens + RT_TOKENS - 1) / RT_TOKENS) * L->experts <= RP_MAX_COUNTS;

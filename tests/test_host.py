@@ -318,4 +318,12 @@ def test_launches_of_a_layer_call():
     layer = C.LayerDesc()
     layer.hidden, layer.ffn, layer.experts, layer.top_k = 4096, 14336, 8, 2
     n = lambda tokens: C.lib.b200moe_layer_launches(ctypes.byref(layer), tokens)
-    assert [n(t) for t in (0, 1, 128, 129, 8192, 8193)] == [0, 4, 4, 5, 5, 6]
+    # 129 tokens and more of long rows: a router CTA per token, plan and permutation until
+    # the two-kernel front has CTAs enough
+    assert [n(t) for t in (0, 1, 128, 129, 353, 354, 8192, 8193)] == [0, 4, 4, 6, 6, 5, 5, 6]
+    layer.hidden, layer.experts = 512, 64
+    assert [n(t) for t in (128, 129, 1024, 1025)] == [4, 5, 5, 6]
+    layer.hidden = 8192
+    assert [n(t) for t in (512, 513, 1025)] == [6, 5, 6]
+    layer.hidden = 16384  # no CTA per token for rows this long
+    assert [n(t) for t in (129, 513)] == [5, 5]
