@@ -135,6 +135,14 @@ int g_token_tile = 192;
 // 252 / 239 (hidden 2048, ffn 4096: 65 / 57; hidden 6144, ffn 16384: 419 / 395).
 constexpr int TENSOR_MIN_TOKENS = 32;
 constexpr int TENSOR_MIN_TOKENS_Q4 = 24;
+// A gate/up product of few rows: its 128-row tiles reach only half of the SMs, the
+// streaming kernel's items are half as high.  8 experts, top 2, gate/up alone, us, stream /
+// tensor, 32 / 48 / 64 / 80 tokens: ffn 1024, hidden 2048 Q8_0 12.2 / 15.2, 12.7 / 15.5,
+// 14.2 / 15.8, 16.7 / 15.6, Q4_K 12.7 / 15.4, 13.3 / 15.5, 14.7 / 15.8, 18.4 / 15.7; ffn 512,
+// hidden 512 6.1 / 7.4, 6.7 / 7.5, 7.3 / 7.4, 8.3 / 7.5.  With top 4 the experts have twice the
+// rows (whole call, 48 / 64 tokens 37 / 36, 46 / 36): between the two.  With twice the tiles
+// (ffn 2048, hidden 1024) 13.4 / 12.6 at 32 tokens already.
+constexpr int TENSOR_MIN_TOKENS_FEW_TILES = 56;
 
 }  // namespace
 
@@ -147,7 +155,8 @@ int pick_regime(int regime, const b200moe_weight_t* w, int max_segment, bool dow
   if (regime == B200MOE_REGIME_STREAM) return B200MOE_REGIME_STREAM;
   const bool can_tensor = w != nullptr && tc_supported(w, down);
   if (!can_tensor) return B200MOE_REGIME_STREAM;
-  const int least = w->layout == B200MOE_LAYOUT_Q4_K && w->experts >= 4 ? TENSOR_MIN_TOKENS_Q4 : TENSOR_MIN_TOKENS;
+  int least = w->layout == B200MOE_LAYOUT_Q4_K && w->experts >= 4 ? TENSOR_MIN_TOKENS_Q4 : TENSOR_MIN_TOKENS;
+  if (!down && 2ll * w->experts * w->rows <= 128ll * sm_count()) least = TENSOR_MIN_TOKENS_FEW_TILES;
   return max_segment >= least ? B200MOE_REGIME_TENSOR : B200MOE_REGIME_STREAM;
 }
 

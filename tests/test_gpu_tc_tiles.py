@@ -94,16 +94,36 @@ def test_prefill_front_routes_as_the_oracle(experts, top_k, tokens, act_dtype):
 
 # one token to each side of where the tensor kernel takes over: 32, and 24 for 4-bit stacks
 # of four or more experts
-@pytest.mark.parametrize("kind,experts,first", [(syn.Q8_0, 8, 32), (syn.Q4_K, 8, 24), (syn.Q4_K, 2, 32)])
+@pytest.mark.parametrize("kind,experts,ffn,first", [(syn.Q8_0, 8, 2048, 32), (syn.Q4_K, 8, 2048, 24),
+                                                    (syn.Q4_K, 2, 5120, 32)])
 @pytest.mark.parametrize("tokens", [23, 24, 31, 32])
-def test_change_over_between_the_kernels(kind, experts, first, tokens):
+def test_change_over_between_the_kernels(kind, experts, ffn, first, tokens):
     from shark_platform_b200 import moe
 
-    spec = syn.CaseSpec("change", tokens, 512, 1024, experts, 2, kind=kind, norm_weight="perturbed", seed=75)
+    spec = syn.CaseSpec("change", tokens, 512, ffn, experts, 2, kind=kind, norm_weight="perturbed", seed=75)
     case = syn.make_case(spec)
     h = device_input(case)
     got = b200_block(case)(h)
     assert torch.equal(got, b200_block(case, regime="tensor" if tokens >= first else "stream")(h))
+    assert moe.device_status() == 0
+    want, _ = orc.moe_block(case.h, oracle_params(case), form="per_expert")
+    assert orc.rel_l2(got.float().cpu(), want) < 2e-2
+
+
+# gate/up rows for half of the SMs or fewer: the streaming kernel up to 55 tokens, beside a
+# down product on the tensor kernel from 32 (24) on
+@pytest.mark.parametrize("kind", [syn.Q8_0, syn.Q4_K])
+@pytest.mark.parametrize("tokens", [23, 32, 48, 55, 56])
+def test_change_over_of_few_row_tiles(kind, tokens):
+    from shark_platform_b200 import moe
+
+    spec = syn.CaseSpec("few_tiles", tokens, 512, 1024, 8, 2, kind=kind, norm_weight="perturbed", router_bias="zipf",
+                        seed=76)
+    case = syn.make_case(spec)
+    h = device_input(case)
+    got = b200_block(case)(h)
+    if tokens in (23, 56):
+        assert torch.equal(got, b200_block(case, regime="tensor" if tokens == 56 else "stream")(h))
     assert moe.device_status() == 0
     want, _ = orc.moe_block(case.h, oracle_params(case), form="per_expert")
     assert orc.rel_l2(got.float().cpu(), want) < 2e-2

@@ -327,3 +327,23 @@ def test_launches_of_a_layer_call():
     assert [n(t) for t in (512, 513, 1025)] == [6, 5, 6]
     layer.hidden = 16384  # no CTA per token for rows this long
     assert [n(t) for t in (129, 513)] == [5, 5]
+
+
+def test_few_gate_up_tiles_stay_on_the_streaming_kernel():
+    """ffn 1024 x 8 experts are 64 tiles of 128 rows on 148 SMs: 56 tokens instead of 32; the
+    down product has its own rule."""
+    import ctypes
+
+    from shark_platform_b200 import _cabi as C
+
+    how = (ctypes.c_int32 * 4)()
+    for ffn, layout, gate, down in ((1024, C.LAYOUT_Q8_0, 56, 32), (1024, C.LAYOUT_Q4_K, 56, 24),
+                                    (1280, C.LAYOUT_Q8_0, 32, 32), (1280, C.LAYOUT_Q4_K, 24, 24)):
+        layer = C.LayerDesc()
+        layer.hidden, layer.ffn, layer.experts, layer.top_k = 2048, ffn, 8, 2
+        layer.gate = layer.up = _desc(layout, 8, ffn, 2048)
+        layer.down = _desc(layout, 8, 2048, ffn)
+        for n in range(1, 120):
+            assert C.lib.b200moe_ep_products(ctypes.byref(layer), C.REGIME_AUTO, n, how) == 0
+            assert how[0] == (C.REGIME_TENSOR if n >= gate else C.REGIME_STREAM)
+            assert how[2] == (C.REGIME_TENSOR if n >= down else C.REGIME_STREAM)
